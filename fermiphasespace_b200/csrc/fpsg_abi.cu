@@ -7,10 +7,12 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <memory>
 #include <string>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "../../include/fpsg.h"
@@ -32,6 +34,7 @@ struct DevAlloc {
 
 template <typename R>
 struct DevTables {
+    void* block = nullptr;  // the device block all of the tables are in
     int *hp = nullptr, *hk = nullptr, *up = nullptr, *uk = nullptr, *vp = nullptr, *vk = nullptr;
     R *tv = nullptr, *xv = nullptr;   // tM_kj and extPot_kj at the entries of hv (energies)
     R *hv = nullptr, *tdiag = nullptr, *ediag = nullptr, *uv = nullptr, *vv = nullptr, *proj = nullptr;
@@ -46,6 +49,9 @@ struct DevTables {
     R* cell_v = nullptr;
     int cell_w = 0;         // 5, 9, 13 or 17; 0 when a column has more than 17 entries
     bool cell_f32 = false;  // every compact weight is exactly an FP32 number
+    int pat_ns = 0;         // offset pattern of Delta (resident path): 2 or 3 offsets, 0 = none
+    Pattern<R> pat = {};
+    R *ud = nullptr, *vd = nullptr;   // dense U, V (long rows), else null
     R* udiag = nullptr;     // U_jj (0 where row j of U has no entry)
     bool dd_fusable = false;  // no Coulomb term, or on-site only (U diagonal): the resident
                               // pass can form the next stage's Delta_jj itself
@@ -77,8 +83,11 @@ struct fpsg_ctx {
     int n = 0, ne = 0, coul = 0, ext_null = 1;
     bool ext_offdiag = false;              // the static potential has an off-diagonal entry
     std::vector<double> tM, U, V, ext;     // dense real parts, col-major
+    void* order_block = nullptr;           // the device block of the next three
     uint32_t* pij = nullptr;
     uint32_t* res_order = nullptr;         // resident kernel's slot order (see res_slot_order)
+    uint32_t* pair_order = nullptr;        // the pair kernels' (pair_slot_order)
+    int n_pair = 0;                        // its length
     DevTables<double> t64;
     DevTables<float> t32;
     int nnz_h = 0;
@@ -238,14 +247,42 @@ int upload(fpsg_ctx* ctx, T** dst, const std::vector<T>& v)
     return FPSG_OK;
 }
 
+// Several host tables in one device block: one allocation and one copy for all of them
+// (some 25 tables per precision, each its own cudaMalloc and cudaMemcpy, were most of the
+// time of fpsg_set_system on a new context).
+struct TableBlock {
+    struct Piece {
+        const void* src;
+        size_t bytes, off;
+        void** dst;
+    };
+    std::vector<Piece> pieces;
+    size_t total = 0;
+
+    template <typename T>
+    void add(T** dst, const std::vector<T>& v)
+    {
+        const size_t bytes = sizeof(T) * std::max<size_t>(v.size(), 1);
+        pieces.push_back({v.data(), sizeof(T) * v.size(), total, (void**)dst});
+        total += (bytes + 255) & ~size_t(255);
+    }
+    int upload(fpsg_ctx* ctx, void** block)
+    {
+        std::vector<unsigned char> host(total);
+        for (const Piece& p : pieces)
+            if (p.bytes) std::memcpy(host.data() + p.off, p.src, p.bytes);
+        int rc = talloc(ctx, block, total);
+        if (rc) return rc;
+        CK(cudaMemcpy(*block, host.data(), total, cudaMemcpyHostToDevice));
+        for (const Piece& p : pieces) *p.dst = (unsigned char*)*block + p.off;
+        return FPSG_OK;
+    }
+};
+
 template <typename R>
 void free_tables(fpsg_ctx* ctx, DevTables<R>& t)
 {
-    trelease(ctx, t.hp); trelease(ctx, t.hk); trelease(ctx, t.up); trelease(ctx, t.uk); trelease(ctx, t.vp);
-    trelease(ctx, t.tv); trelease(ctx, t.xv);
-    trelease(ctx, t.vk); trelease(ctx, t.hv); trelease(ctx, t.tdiag); trelease(ctx, t.ediag); trelease(ctx, t.uv);
-    trelease(ctx, t.vv); trelease(ctx, t.proj); trelease(ctx, t.ell_k); trelease(ctx, t.ell_v);
-    trelease(ctx, t.ell_pad); trelease(ctx, t.udiag); trelease(ctx, t.cell_k); trelease(ctx, t.cell_v);
+    trelease(ctx, t.block);
     t = DevTables<R>();
 }
 
@@ -404,16 +441,54 @@ int build_tables(fpsg_ctx* ctx, DevTables<R>& t)
     t.cell_f32 = true;
     for (const R v : cv)
         if ((R)(float)v != v) t.cell_f32 = false;
-    int rc;
-    if ((rc = upload(ctx, &t.cell_k, ck)) || (rc = upload(ctx, &t.cell_v, cv))) return rc;
-    if ((rc = upload(ctx, &t.hp, hp)) || (rc = upload(ctx, &t.hk, hk)) || (rc = upload(ctx, &t.hv, hv)) ||
-        (rc = upload(ctx, &t.tv, tvv)) || (rc = upload(ctx, &t.xv, xvv)) ||
-        (rc = upload(ctx, &t.tdiag, tdiag)) || (rc = upload(ctx, &t.ediag, ediag)) ||
-        (rc = upload(ctx, &t.up, up)) || (rc = upload(ctx, &t.uk, uk)) || (rc = upload(ctx, &t.uv, uv)) ||
-        (rc = upload(ctx, &t.vp, vp)) || (rc = upload(ctx, &t.vk, vk)) || (rc = upload(ctx, &t.vv, vv)) ||
-        (rc = upload(ctx, &t.proj, proj)) || (rc = upload(ctx, &t.ell_k, ek)) || (rc = upload(ctx, &t.ell_v, ev)) ||
-        (rc = upload(ctx, &t.ell_pad, t.ell_dpad)) || (rc = upload(ctx, &t.udiag, udiag)))
-        return rc;
+    // offset pattern: the distinct |k - j| of Delta's off-diagonal nonzeros, descending to
+    // 1, when there are at most PAT_MAX and one value throughout.  A pattern with fewer
+    // than two offsets is filled up in front with one that no column uses.
+    std::vector<int> offs;
+    bool pat_ok = true;
+    for (int j = 0; j < n && pat_ok; ++j)
+        for (int q = hp[j]; q < hp[j + 1] && pat_ok; ++q) {
+            if (hk[q] <= j) continue;                       // Delta is symmetric
+            if (offs.empty()) t.pat.w = hv[q];
+            if (std::find(offs.begin(), offs.end(), hk[q] - j) == offs.end()) offs.push_back(hk[q] - j);
+            pat_ok = hv[q] == t.pat.w && (int)offs.size() <= PAT_MAX;
+        }
+    std::sort(offs.begin(), offs.end(), std::greater<int>());
+    if (offs.empty() || offs.back() != 1) offs.push_back(1);
+    while (offs.size() < 2) offs.insert(offs.begin(), 1);
+    std::vector<uint32_t> pmask(n, 0u);
+    if (pat_ok && (int)offs.size() <= PAT_MAX) {
+        t.pat_ns = (int)offs.size();
+        for (int s2 = 0; s2 < t.pat_ns; ++s2) t.pat.off[s2] = offs[s2];
+        for (int j = 0; j < n; ++j)
+            for (int q = hp[j]; q < hp[j + 1]; ++q) {
+                if (hk[q] == j) continue;
+                int o = t.pat_ns - 1;
+                while (t.pat.off[o] != std::abs(hk[q] - j)) --o;
+                pmask[j] |= 1u << (2 * o + (hk[q] > j ? 1 : 0));
+            }
+    }
+    // dense rows of U (and V) where most of their entries are nonzero
+    std::vector<R> ud, vd;
+    const size_t nn = (size_t)n * n;
+    if (ctx->coul != FPSG_COULOMB_NULL && 2 * (uk.size() + (ctx->coul == FPSG_COULOMB_DISTANCE ? vk.size() : 0)) >= nn && n > 4) {
+        ud.resize(nn);
+        vd.resize(nn);
+        for (size_t q = 0; q < nn; ++q) { ud[q] = (R)ctx->U[q]; vd[q] = (R)ctx->V[q]; }
+    }
+    TableBlock tb;
+    uint32_t* d_mask = nullptr;
+    tb.add(&d_mask, pmask);
+    if (!ud.empty()) { tb.add(&t.ud, ud); tb.add(&t.vd, vd); }
+    tb.add(&t.cell_k, ck); tb.add(&t.cell_v, cv);
+    tb.add(&t.hp, hp); tb.add(&t.hk, hk); tb.add(&t.hv, hv); tb.add(&t.tv, tvv); tb.add(&t.xv, xvv);
+    tb.add(&t.tdiag, tdiag); tb.add(&t.ediag, ediag); tb.add(&t.proj, proj); tb.add(&t.udiag, udiag);
+    tb.add(&t.up, up); tb.add(&t.uk, uk); tb.add(&t.uv, uv);
+    tb.add(&t.vp, vp); tb.add(&t.vk, vk); tb.add(&t.vv, vv);
+    tb.add(&t.ell_k, ek); tb.add(&t.ell_v, ev); tb.add(&t.ell_pad, t.ell_dpad);
+    const int rc = tb.upload(ctx, &t.block);
+    if (rc) return rc;
+    t.pat.mask = d_mask;
     return FPSG_OK;
 }
 
@@ -424,6 +499,7 @@ DevSys<R> make_sys(fpsg_ctx* ctx, const DevTables<R>& t, int method)
     s.n = ctx->n; s.ne = ctx->ne;
     s.hp = t.hp; s.hk = t.hk; s.hv = t.hv; s.tv = t.tv; s.xv = t.xv; s.tdiag = t.tdiag; s.ediag = t.ediag;
     s.up = t.up; s.uk = t.uk; s.uv = t.uv; s.vp = t.vp; s.vk = t.vk; s.vv = t.vv;
+    s.ud = t.ud; s.vd = t.vd;
     s.pij = ctx->pij;
     s.coul = ctx->coul;
     s.fock = (method == FPSG_METHOD_HF && ctx->coul == FPSG_COULOMB_DISTANCE) ? 1 : 0;
@@ -455,52 +531,66 @@ struct ResPlan {
     int idx = -1, G = 0;
     size_t smem = 0;
     bool comp = false;   // FP32 compensated state update (state read and written in FP64)
+    bool pair = false;   // k_pair (idx into pair_cfgs)
+    bool coul_smem = false;   // with pair: dense U and V in shared memory
     bool quad = false;   // k_resident_quad (4-CTA clusters, idx into quad_cfgs), G = 1
     bool hp = false;     // with quad: k_resident_quad_hp (idx into quad_hp_cfgs)
     bool e8 = false;     // with hp: 8-byte column entries (FP32 weights)
     int nh = 2;          // with hp: CTAs per spin (1: 2-CTA clusters)
 };
 
-template <typename R>
-size_t res_bytes(int n, int M, int P, int cap, bool comp = false)
-{
-    return res_layout_direct<R>(n, M, P, cap, comp).total;
-}
-
 // Picks a resident configuration and the trajectories per CTA: the stacked rows
 // (M n) fill whole warps, the elements fit the thread x register budget, the
 // shared memory fits, and there are enough CTAs to cover the SMs.
 template <typename R>
-ResPlan plan_resident(fpsg_ctx* ctx, int B, bool comp = false)
+ResPlan plan_resident_of(fpsg_ctx* ctx, int B, bool comp, bool pair)
 {
     ResPlan best;
-    const auto& cf = res_cfgs<R>();
+    const auto& cf = pair ? pair_cfgs<R>() : res_cfgs<R>();
     const int n = ctx->n, ne = ctx->ne;
-    const int P = tables<R>(ctx).ell_p;
+    const DevTables<R>& t = tables<R>(ctx);
+    const int items = pair ? ctx->n_pair : ne;      // slots or elements per matrix
     double best_score = -1e300;
-    if (P == 0) return best;      // a column too wide for the fixed-width stencil
+    if (pair ? (t.pat_ns == 0 || n > PAIR_NMAX) : t.ell_p == 0) return best;
     for (int c = 0; c < (int)cf.size(); ++c) {
         const int per = cf[c].split ? 1 : 2;
         const int cap = cf[c].nt * cf[c].ept;
-        int Gmax = cap / (per * ne);
-        while (Gmax > 0 && res_bytes<R>(n, per * Gmax, P, cap, comp) > ctx->smem_optin) --Gmax;
+        auto bytes = [&](int G, bool uv = false) {
+            return pair ? pair_layout<R>(n, per * G, cap, comp, t.pat.off[0], t.ud != nullptr, uv).total
+                        : res_layout_direct<R>(n, per * G, t.ell_p, cap, comp, t.ud != nullptr).total;
+        };
+        int Gmax = std::min(cap / (per * items), PAIR_MMAX / per);
+        while (Gmax > 0 && bytes(Gmax) > ctx->smem_optin) --Gmax;
         if (Gmax < 1) continue;
         const int ctas_per_group = cf[c].split ? 2 : 1;
         const int want_groups = std::max(1, ctx->sm_count * 2 / ctas_per_group);
         int G = std::max(1, std::min(Gmax, (B + want_groups - 1) / want_groups));
         const int M = per * G;
-        const double elem_fill = (double)(M * ne) / cap;                          // thread utilisation
+        const double elem_fill = (double)(M * items) / cap;                       // thread utilisation
         const double row_fill = (double)(M * n) / (32.0 * ((M * n + 31) / 32));     // lane utilisation
         const double split_pen = cf[c].split ? 0.9 : 1.0;
-        const double score = elem_fill * row_fill * split_pen - 0.002 * cf[c].ept;
+        const double score = elem_fill * row_fill * split_pen - 0.002 * cf[c].ept * (pair ? 2 : 1);
         if (score > best_score) {
             best_score = score;
             best.idx = c; best.G = G;
-            best.smem = res_bytes<R>(n, M, P, cap, comp);
+            best.pair = pair;
+            best.coul_smem = pair && t.ud != nullptr && bytes(G, true) <= ctx->smem_optin;
+            best.smem = bytes(G, best.coul_smem);
             best.comp = comp;
         }
     }
     return best;
+}
+
+// The pair kernels wherever Delta has an offset pattern and a configuration fits: they
+// need fewer shared-memory wavefronts per element than the column kernels at every P
+// such a Delta can have (fpsg_pair.cuh), also where half of the slots is masked
+// (three offsets and three neighbours per site, as the honeycomb lattice has).
+template <typename R>
+ResPlan plan_resident(fpsg_ctx* ctx, int B, bool comp = false)
+{
+    const ResPlan plan = plan_resident_of<R>(ctx, B, comp, true);
+    return plan.idx < 0 ? plan_resident_of<R>(ctx, B, comp, false) : plan;
 }
 
 // The 4-CTA-cluster kernel for matrices too large for k_resident: the smallest
@@ -568,6 +658,7 @@ int set_error_from_flag(fpsg_ctx* ctx, unsigned flag)
 {
     if (flag & 1u) return fail(ctx, FPSG_ERR_DIVERGED, "a trajectory became non-finite");
     if (flag & (1u << 4)) return fail(ctx, FPSG_ERR_TIMEOUT, "a device-side wait of the dense path gave up");
+    if (flag & ERR_PEER_WAIT) return fail(ctx, FPSG_ERR_TIMEOUT, "a device-side wait for a cluster's peer gave up");
     return FPSG_OK;
 }
 
@@ -617,8 +708,9 @@ struct ResLauncher {
             grid = cdim * std::min(B, ncl);
             return FPSG_OK;
         }
-        const ResCfg<R>& cfg = res_cfgs<R>()[plan.idx];
-        fn = dump ? cfg.fn_dump[p_index(tables<R>(ctx).ell_p)] : cfg.fn[p_index(tables<R>(ctx).ell_p)];
+        const ResCfg<R>& cfg = (plan.pair ? pair_cfgs<R>() : res_cfgs<R>())[plan.idx];
+        const int v = plan.pair ? tables<R>(ctx).pat_ns - 2 : p_index(tables<R>(ctx).ell_p);
+        fn = dump ? cfg.fn_dump[v] : cfg.fn[v];
         nt = cfg.nt; split = cfg.split; cdim = split ? 2 : 1; smem = plan.smem;
         CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         const int ngroups = (B + plan.G - 1) / plan.G;
@@ -766,11 +858,12 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
         ra.record = q.record; ra.do_en = rec_e; ra.do_e1 = do_e1 && rec_e; ra.do_e2 = do_e2 && rec_e;
         ra.ell_k = plan.quad ? tables<R>(ctx).cell_k : tables<R>(ctx).ell_k;
         ra.ell_v = plan.quad ? tables<R>(ctx).cell_v : tables<R>(ctx).ell_v;
-        ra.ell_pad = tables<R>(ctx).ell_pad;
+        ra.ell_pad = tables<R>(ctx).ell_pad; ra.pat = tables<R>(ctx).pat;
         ra.slots = slots; ra.whole = whole; ra.err = d_err;
         ra.dump = nullptr; ra.dump_count = 0;
         ra.udiag = tables<R>(ctx).dd_fusable ? tables<R>(ctx).udiag : nullptr;
-        ra.order = ctx->res_order;
+        ra.order = plan.pair ? ctx->pair_order : ctx->res_order; ra.nslots = ctx->n_pair;
+        ra.coul_smem = plan.coul_smem ? 1 : 0;
         ra.state64 = plan.comp ? ctx->rho64 : nullptr;
         // chunk the time axis so one launch stays in the tens of milliseconds
         const long per_launch_steps = std::max<long>(1, 4096L * 1024 / std::max<long>(1, (long)B));
@@ -1268,10 +1361,12 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
         ra.sys = sys; ra.state = st; ra.B = B; ra.G = plan.G; ra.h = (R)h;
         ra.S = S; ra.Tp = Tp; ra.hf = 1; ra.record = 1; ra.do_en = 0; ra.do_e1 = 0; ra.do_e2 = 0;
         ra.ell_k = tables<R>(ctx).ell_k; ra.ell_v = tables<R>(ctx).ell_v; ra.ell_pad = tables<R>(ctx).ell_pad;
+        ra.pat = tables<R>(ctx).pat;
         ra.slots = slots; ra.whole = nullptr; ra.err = d_err; ra.step_base = 0;
         ra.dump = nullptr; ra.dump_count = 0;
         ra.udiag = tables<R>(ctx).dd_fusable ? tables<R>(ctx).udiag : nullptr;
-        ra.order = ctx->res_order;
+        ra.order = plan.pair ? ctx->pair_order : ctx->res_order; ra.nslots = ctx->n_pair;
+        ra.coul_smem = plan.coul_smem ? 1 : 0;
         // The last n_keep segments of a chunk keep their stage inputs from its sweep
         // (the recompute variant of the kernel, records on), so the backward pass needs
         // no recompute for them: in whole segments, up to three quarters of the free
@@ -1734,10 +1829,11 @@ int batch_impl(fpsg_ctx* ctx, const fpsg_system_desc* sd, int ns, int method, do
         ra.do_e2 = (hf ? (c->coul == FPSG_COULOMB_DISTANCE) : 1) && rec_e;
         ra.ell_k = plan.quad ? tables<R>(c).cell_k : tables<R>(c).ell_k;
         ra.ell_v = plan.quad ? tables<R>(c).cell_v : tables<R>(c).ell_v;
-        ra.ell_pad = tables<R>(c).ell_pad;
+        ra.ell_pad = tables<R>(c).ell_pad; ra.pat = tables<R>(c).pat;
         ra.slots = r.slots; ra.whole = nullptr; ra.err = d_err; ra.dump = nullptr; ra.dump_count = 0;
         ra.udiag = tables<R>(c).dd_fusable ? tables<R>(c).udiag : nullptr;
-        ra.order = c->res_order;
+        ra.order = plan.pair ? c->pair_order : c->res_order; ra.nslots = c->n_pair;
+        ra.coul_smem = plan.coul_smem ? 1 : 0;
         ra.state64 = plan.comp ? c->rho64 : nullptr;
         path_of[k] = FPSG_PATH_RESIDENT;
         rs.push_back(r);
@@ -2075,8 +2171,8 @@ int fpsg_set_system(fpsg_ctx* ctx, int n, const double* tM, const double* U, con
     if (cudaSetDevice(ctx->device) != cudaSuccess) return fail(ctx, FPSG_ERR_CUDA, "cudaSetDevice");
     free_tables(ctx, ctx->t64);
     free_tables(ctx, ctx->t32);
-    trelease(ctx, ctx->pij); ctx->pij = nullptr;
-    trelease(ctx, ctx->res_order); ctx->res_order = nullptr;
+    trelease(ctx, ctx->order_block); ctx->order_block = nullptr;
+    ctx->pij = ctx->res_order = ctx->pair_order = nullptr;
     if (ctx->B > 0 && ctx->n != n) { dfree(ctx, ctx->rho64); ctx->rho64 = nullptr; ctx->B = 0; }
     ctx->n = n;
     ctx->ne = n * (n + 1) / 2;
@@ -2099,7 +2195,11 @@ int fpsg_set_system(fpsg_ctx* ctx, int n, const double* tM, const double* U, con
     for (int j = 0; j < n; ++j)
         for (int i = 0; i <= j; ++i) pij[(size_t)cs(j) + i] = (uint32_t)i | ((uint32_t)j << 16);
     int rc;
-    if ((rc = upload(ctx, &ctx->pij, pij)) || (rc = upload(ctx, &ctx->res_order, res_slot_order(n)))) return rc;
+    const std::vector<uint32_t> ro = res_slot_order(n), po = pair_slot_order(n);
+    ctx->n_pair = (int)po.size();
+    TableBlock tb;
+    tb.add(&ctx->pij, pij); tb.add(&ctx->res_order, ro); tb.add(&ctx->pair_order, po);
+    if ((rc = tb.upload(ctx, &ctx->order_block))) return rc;
     if ((rc = build_tables<double>(ctx, ctx->t64))) return rc;
     if ((rc = build_tables<float>(ctx, ctx->t32))) return rc;
     ctx->sys_set = true;

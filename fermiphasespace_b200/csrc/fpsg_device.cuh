@@ -84,6 +84,8 @@ struct DevSys {
     const R* ediag;    // extPot_jj (static potential), 0 when absent
     const int* up; const int* uk; const R* uv;   // U by rows (nonzeros)
     const int* vp; const int* vk; const R* vv;   // V by rows (nonzeros), coulomb == DISTANCE
+    // U and V as dense [n][n] when their rows are long (symmetric, so rows are columns); else null
+    const R* ud; const R* vd;
     const uint32_t* pij;  // packed index -> i | (j << 16)
     int coul;       // 0 null, 1 onSite, 2 distance
     int fock;       // HF with distance Coulomb: Delta has the exchange term -N o V

@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(256) k_stream_record(StreamArgs<R> a)
 //   dg  [2][M n + 1]                diagonal of X, double-buffered like X; the
 //                                   other spin (possibly in the peer CTA) reads it
 //                                   for its Hartree term
-//   es  [M][4] double               energy partials
+//   es  [32][4] double              energy partials per warp
 //   ell [2P+1][n]                   Delta's column j as fixed-width entries, slot-major
 //                                   (lanes reading column i of consecutive i hit
 //                                   consecutive entries)
@@ -348,6 +348,20 @@ __global__ void __launch_bounds__(256) k_stream_record(StreamArgs<R> a)
 // element X(m; j, i) of consecutive i) fall in distinct banks; the spare slot at
 // n*RP absorbs the writes of threads that have no element, so the hot loop has no
 // branches.
+
+// Offset pattern of Delta off its diagonal: every nonzero Delta_kj has k - j = +-off[q]
+// and the value w, and bit 2q (2q + 1) of mask[j] says whether row j - off[q]
+// (j + off[q]) exists in column j.  Offsets descend to 1, so the slots 0, 2, 4 are the
+// rows below j in ascending order and 5, 3, 1 those above it.  Lattices numbered row by
+// row have one (a grid: nx, 1; in 3D: nx ny, nx, 1).
+constexpr int PAT_MAX = 3;
+template <typename R>
+struct Pattern {
+    const uint32_t* mask;
+    int off[PAT_MAX];
+    R w;
+};
+
 template <typename R>
 struct ResArgs {
     DevSys<R> sys;
@@ -364,6 +378,8 @@ struct ResArgs {
     double* slots;        // [gridDim.x][Tp][W]
     double2* whole;       // [Tp][2][ne] or null
     unsigned* err;
+    int coul_smem = 0;    // pair kernels: dense U and V copied to shared memory
+    int nslots = 0;       // pair kernels: slots per matrix (order holds pair_slot_order)
     // optional: every step's four stage inputs, [step][4][B][2][ne] packed (the
     // adjoint's segment recompute); null = not kept
     cplx<R>* dump;
@@ -381,6 +397,8 @@ struct ResArgs {
     // the rounding residual of the last update (a bf16 pair in shared memory), and
     // hi + lo goes back to FP64 at the end of the launch
     cplx<double>* state64 = nullptr;
+    // offset pattern of Delta (pair kernels)
+    Pattern<R> pat = {};
 };
 
 // bf16 pair <-> float pair (low half = first value); bf16 -> float is exact
@@ -415,6 +433,95 @@ __device__ __forceinline__ void rk_final_comp(cplx<float> k, float h, cplx<float
     lo2 = pack_bf16x2(rre, rim);
 }
 
+// Complex FP32 values as register pairs for the two-wide FP32 instructions of sm_100
+// (each component rounded as the scalar instruction rounds it).
+__device__ __forceinline__ uint64_t f2_pack(float a, float b)
+{
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+    return v;
+}
+__device__ __forceinline__ cplx<float> f2_unpack(uint64_t v)
+{
+    cplx<float> x;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x.re), "=f"(x.im) : "l"(v));
+    return x;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b)
+{
+    uint64_t v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ uint64_t f2_sub(uint64_t a, uint64_t b)
+{
+    uint64_t v;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+// acc += x where `code` has `BIT` set
+template <uint32_t BIT>
+__device__ __forceinline__ void f2_add_if(uint64_t& acc, uint64_t x, uint32_t code)
+{
+    asm("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\tand.b32 t, %2, %3;\n\tsetp.ne.u32 p, t, 0;\n\t"
+        "@p add.rn.f32x2 %0, %0, %1;\n\t}"
+        : "+l"(acc) : "l"(x), "r"(code), "n"(BIT));
+}
+// c x + y, componentwise (scalar instructions: they take a constant as an operand, the
+// two-wide ones would need it in a register pair)
+__device__ __forceinline__ uint64_t f2_axpy(float c, uint64_t x, uint64_t y)
+{
+    const cplx<float> u = f2_unpack(x), v = f2_unpack(y);
+    return f2_pack(__fmaf_rn(u.re, c, v.re), __fmaf_rn(u.im, c, v.im));
+}
+// rho + hs k with k = -i g: (g.im, -g.re) scaled
+__device__ __forceinline__ uint64_t f2_step(uint64_t rho, uint64_t g, float hs)
+{
+    const cplx<float> r = f2_unpack(rho), x = f2_unpack(g);
+    return f2_pack(__fmaf_rn(x.im, hs, r.re), __fmaf_rn(x.re, -hs, r.im));
+}
+
+// The RK stages of the FP32 pair pass, in terms of g = i k (so that no components
+// are swapped before the update).  a, b hold g1, g2 up to stage 3 instead of rk_update's
+// combinations: a thread then forms its own element of the stage input from registers
+// and the state it reads anyway, instead of loading it from X.
+//     X2 = rho + h/3 k1,  X3 = rho + h (k2 - k1/3),  X4 = rho + h ((k1 - k2) + k3),
+//     rho' = rho + h/8 (((k1 + 3 k2) + 3 k3) + k4)
+__device__ __forceinline__ uint64_t f2_stage_input(int stage, uint64_t rho, uint64_t a, uint64_t b, float h)
+{
+    if (stage == 0) return rho;
+    if (stage == 1) return f2_step(rho, a, h * (1.0f / 3.0f));
+    if (stage == 2) return f2_step(rho, f2_axpy(-1.0f / 3.0f, a, b), h);
+    return f2_step(rho, a, h);                 // a = (g1 - g2) + g3 by then
+}
+__device__ __forceinline__ uint64_t f2_stage(int stage, uint64_t rho, uint64_t g, uint64_t& a, uint64_t& b, float h)
+{
+    if (stage == 0) {
+        a = g;
+    } else if (stage == 1) {
+        b = g;
+    } else {
+        const uint64_t g1 = a, g2 = b;
+        a = f2_add(f2_sub(g1, g2), g);
+        b = f2_axpy(3.0f, g, f2_axpy(3.0f, g2, g1));
+    }
+    return f2_stage_input(stage + 1, rho, a, b, h);
+}
+// the last stage, with the compensated state update of rk_final_comp (comp)
+__device__ __forceinline__ uint64_t f2_final(uint64_t rho, uint64_t g, uint64_t b, float h, bool comp, uint32_t& lo2)
+{
+    const float hs = h * 0.125f;
+    const uint64_t s = f2_add(b, g);
+    if (!comp) return f2_step(rho, s, hs);
+    const float2 lo = unpack_bf16x2(lo2);
+    const uint64_t d = f2_step(f2_pack(lo.x, lo.y), s, hs);
+    const uint64_t sum = f2_add(rho, d);
+    const uint64_t bb = f2_sub(sum, rho);
+    const cplx<float> r = f2_unpack(f2_add(f2_sub(rho, f2_sub(sum, bb)), f2_sub(d, bb)));
+    lo2 = pack_bf16x2(r.re, r.im);
+    return sum;
+}
+
 // where a resident element's value goes in a packed [B][2][ne] buffer
 struct DumpMap {
     int gbase, rank, B, ne, split;
@@ -435,7 +542,7 @@ __host__ __device__ __forceinline__ size_t align16(size_t x) { return (x + 15) &
 
 template <typename R>
 struct ResLayout {
-    size_t x, rho, dd, dg, es, ell, lo, xs, sd, total;
+    size_t x, rho, dd, dg, es, ell, lo, xs, sd, uv, total;
 };
 
 // Delta_jj from diagonal arrays (same spin, other spin), order as delta_diag.
@@ -460,38 +567,203 @@ __device__ __forceinline__ R delta_diag_v(const DevSys<R>& s, int j, const R* sa
     return d;
 }
 
-// energy partials of one matrix in the stacked layout (see energy_partials)
+// Delta_jj of the RR = M n (matrix, site) items of a CTA, followed by a block barrier.
+// Sparse Coulomb rows: one thread per item (delta_diag_v).  Dense ones (sys.ud, a distance
+// interaction): column-major U and V (ud, vd: in shared memory where it has room), so that
+// the threads of a warp read consecutive columns j of the same row k.  FP32 splits each
+// sum over k among the threads the CTA has to spare and, with both spins in the CTA (BOTH),
+// takes both spins' sums from one read of U and V.  FP64 keeps the oracle's order,
+// ascending k in one chain per term, the U and the V sum of an item on two threads.
+// The CSR rows (index, weight and density one after the other, one thread per item) took
+// 14 K of the 24 K cycles of a stage at 63 sites, FP32, both spins in the CTA; this takes
+// 3 K.
 template <typename R>
-__device__ __forceinline__ void energy_partials_full(const DevSys<R>& s, const cplx<R>* X, int RP, int row0,
-                                                     const R* dsame, const R* dother, int spin, int do_e1,
-                                                     int do_e2, int lane, int nlanes, double e[4])
+__host__ __device__ __forceinline__ size_t coul_scratch(int RR)
+{
+    const size_t two = 2 * (size_t)RR;
+    return std::is_same<R, float>::value && two < 1024 ? 1024 : two;
+}
+template <typename R, int NT, bool BOTH, typename SAME, typename OTHER>
+__device__ __forceinline__ void delta_diag_block(const DevSys<R>& s, const R* ud, const R* vd, R* Dc, R* scr, int RR,
+                                                 SAME same, OTHER other, R pulse, int tid)
+{
+    const int n = s.n;
+    if (s.ud == nullptr) {
+        for (int w = tid; w < RR; w += NT) {
+            const int m = w / n, j = w - m * n;
+            Dc[w] = delta_diag_v<R>(s, j, same(m), other(m), pulse);
+        }
+        __syncthreads();
+        return;
+    }
+    const bool v_on = s.coul == 2;
+    constexpr int SP = BOTH ? 2 : 1;                     // sums per item
+    const int items = RR / SP;
+    int parts = 1;                                       // FP32: pieces of each sum over k
+    if constexpr (std::is_same<R, float>::value) {
+        while (2 * parts * items <= NT && parts < 8) parts *= 2;
+        const int len = (n + parts - 1) / parts;
+        for (int w = tid; w < parts * items; w += NT) {
+            const int p = w / items, x = w - p * items, g = x / n, j = x - g * n;
+            const R* o = other(SP * g);                  // the other spin of matrix SP g
+            const R* e = same(SP * g);
+            const int k0 = p * len, k1 = min(n, k0 + len);
+            R a0 = R(0), a1 = R(0);
+#pragma unroll 4
+            for (int k = k0; k < k1; ++k) {
+                const R u = ud[k * n + j], v = v_on ? vd[k * n + j] : R(0);
+                const R no = o[k] + s.shift, ne = e[k] + s.shift;
+                a0 = fmaR<R>(u, no, fmaR<R>(v, ne, a0));
+                if (BOTH) a1 = fmaR<R>(u, ne, fmaR<R>(v, no, a1));
+            }
+            scr[(p * SP) * items + x] = a0;
+            if (BOTH) scr[(p * SP + 1) * items + x] = a1;
+        }
+    } else {
+        for (int w = tid; w < (v_on ? 2 : 1) * RR; w += NT) {
+            const bool vt = w >= RR;
+            const int x = vt ? w - RR : w, m = x / n, j = x - m * n;
+            const R* d = vt ? same(m) : other(m);
+            const R* c = (vt ? vd : ud) + j;
+            R u = R(0);
+#pragma unroll 8
+            for (int k = 0; k < n; ++k) u = fmaR<R>(c[k * n], addR<R>(d[k], s.shift), u);
+            scr[w] = u;
+        }
+    }
+    __syncthreads();
+    for (int w = tid; w < RR; w += NT) {
+        const int m = w / n, j = w - m * n;
+        R d = s.tdiag[j];
+        if constexpr (std::is_same<R, float>::value) {
+            const int x = (m / SP) * n + j, sp = m % SP;
+            R u = scr[sp * items + x];
+            for (int p = 1; p < parts; ++p) u += scr[(p * SP + sp) * items + x];
+            d += u;
+        } else {
+            d = addR<R>(d, scr[w]);
+            if (v_on) d = addR<R>(d, scr[RR + w]);
+        }
+        if (s.has_ext) d = addR<R>(d, s.ediag[j]);
+        if (s.n_bins > 0) d = addR<R>(d, mulR<R>(pulse, s.proj[j]));
+        Dc[w] = d;
+    }
+    __syncthreads();
+}
+
+// energy terms of site j of one matrix in the stacked layout (see energy_partials).  With
+// dense Coulomb rows the sums over k are split: part p of `parts` takes its share of them
+// (p = 0 the site's other terms too); the caller adds everything up anyway.
+// re(k): Re X(k, j) for a row k of column j of Delta.
+template <typename R, typename RE>
+__device__ __forceinline__ void energy_site(const DevSys<R>& s, int j, RE re, const R* dsame, const R* dother, int spin, int do_e1, int do_e2,
+                                            double e[4], int p = 0, int parts = 1)
 {
     const double shift = (double)s.shift;
-    for (int j = lane; j < s.n; j += nlanes) {
-        const double nj = (double)dsame[j] + shift;
+    const double nj = (double)dsame[j] + shift;
+    if (p == 0) {
         double t0 = nj * (double)s.tdiag[j], t3 = 0.0;
         for (int q = s.hp[j]; q < s.hp[j + 1]; ++q) {
             const int k = s.hk[q];
             if (k == j) continue;
-            const double x = (double)X[j * RP + row0 + k].re;
+            const double x = (double)re(k);
             t0 += x * (double)s.tv[q];
             if (s.has_ext) t3 += x * (double)s.xv[q];
         }
         e[0] += t0;
         if (s.has_ext) e[3] += nj * (double)s.ediag[j] + t3;
-        if (do_e2) {
-            double v = 0.0;
+    }
+    const bool e1 = do_e1 && spin == 0;
+    const double oj = (double)dother[j] + shift;
+    double v = 0.0, uo = 0.0, us = 0.0;
+    if (s.ud != nullptr) {
+        const int len = (s.n + parts - 1) / parts, k1 = min(s.n, (p + 1) * len);
+        if (do_e2)
+#pragma unroll 4
+            for (int k = p * len; k < k1; ++k) v += (double)s.vd[k * s.n + j] * ((double)dsame[k] + shift);
+        if (e1)
+#pragma unroll 4
+            for (int k = p * len; k < k1; ++k) {
+                const double u = (double)s.ud[k * s.n + j];
+                uo += u * ((double)dother[k] + shift);
+                us += u * ((double)dsame[k] + shift);
+            }
+    } else {
+        if (do_e2)
             for (int q = s.vp[j]; q < s.vp[j + 1]; ++q) v += (double)s.vv[q] * ((double)dsame[s.vk[q]] + shift);
-            e[2] += 0.5 * nj * v;
-        }
-        if (do_e1 && spin == 0) {
-            const double oj = (double)dother[j] + shift;
-            double uo = 0.0, us = 0.0;
+        if (e1)
             for (int q = s.up[j]; q < s.up[j + 1]; ++q) {
                 uo += (double)s.uv[q] * ((double)dother[s.uk[q]] + shift);
                 us += (double)s.uv[q] * ((double)dsame[s.uk[q]] + shift);
             }
-            e[1] += 0.5 * (nj * uo + oj * us);
+    }
+    if (do_e2) e[2] += 0.5 * nj * v;
+    if (e1) e[1] += 0.5 * (nj * uo + oj * us);
+}
+
+// energy partials of one matrix, sites lane, lane + nlanes, ...
+template <typename R>
+__device__ __forceinline__ void energy_partials_full(const DevSys<R>& s, const cplx<R>* X, int RP, int row0,
+                                                     const R* dsame, const R* dother, int spin, int do_e1,
+                                                     int do_e2, int lane, int nlanes, double e[4])
+{
+    for (int j = lane; j < s.n; j += nlanes)
+        energy_site<R>(s, j, [&](int k) { return X[j * RP + row0 + k].re; }, dsame, dother, spin, do_e1, do_e2, e);
+}
+
+// One snapshot record of the CTA's matrices: the diagonal sums and, with energies, the
+// four energy rows, added to the CTA's slot.  Every (matrix, site) pair is one thread's
+// item and the CTA sums the energies of all its matrices at once (a loop over the
+// matrices left n of the NT threads working and crossed two block barriers per matrix).
+// re(m, k, j): Re X(k, j) of matrix m.
+template <typename R, int NT, bool SPLIT, typename RE, typename OTHER>
+__device__ __forceinline__ void res_record(const ResArgs<R>& a, RE re, const R* d0, OTHER other,
+                                           double* es, double* slot, int gid, int rank, int tid)
+{
+    const int n = a.sys.n;
+    const int nvec = SPLIT ? (rank == 0 ? 3 : 2) : 5;
+    const int G = min(a.G, a.B - gid * a.G);             // trajectories of this group
+    for (int w = tid; w < nvec * n; w += NT) {
+        const int oo = w / n, j = w - oo * n;
+        int o;
+        if (SPLIT) o = rank == 0 ? (oo == 0 ? 0 : oo == 1 ? 2 : 4) : (oo == 0 ? 1 : 3);
+        else o = oo;
+        double acc = 0.0;
+        for (int g = 0; g < G; ++g) {
+            double du, dd;
+            if (SPLIT) {
+                const double mine = (double)d0[g * n + j], oth = (double)other(g)[j];
+                du = rank == 0 ? mine : oth;
+                dd = rank == 0 ? oth : mine;
+            } else {
+                du = (double)d0[(2 * g) * n + j];
+                dd = (double)d0[(2 * g + 1) * n + j];
+            }
+            if (!isfinite(du) || !isfinite(dd)) atomicOr(a.err, 1u);
+            acc += o == 0 ? du : o == 1 ? dd : o == 2 ? du * du : o == 3 ? dd * dd : du * dd;
+        }
+        atomicAdd(slot + o * n + j, acc);
+    }
+    if (a.do_en) {
+        const int M = SPLIT ? G : 2 * G;
+        double e[4] = {0.0, 0.0, 0.0, 0.0};
+        const int parts = a.sys.ud != nullptr ? min(8, max(1, NT / (M * n))) : 1;
+        for (int w = tid; w < M * n * parts; w += NT) {
+            const int p = w / (M * n), x = w - p * M * n, m = x / n, j = x - m * n;
+            energy_site<R>(a.sys, j, [&](int k) { return re(m, k, j); }, d0 + m * n, other(m), SPLIT ? rank : (m & 1),
+                           a.do_e1, a.do_e2, e, p, parts);
+        }
+        const int lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const double v = warp_sum(e[c]);
+            if (lane == 0) es[warp * 4 + c] = v;
+        }
+        __syncthreads();
+        if (tid < 4) {
+            double v = 0.0;
+            for (int q = 0; q < NT / 32; ++q) v += es[q * 4 + tid];
+            atomicAdd(slot + 5 * n + tid, v);
         }
     }
 }
@@ -505,7 +777,8 @@ __device__ __forceinline__ void energy_partials_full(const DevSys<R>& s, const c
 // both in ascending k (oracle order), then dX_ij = -i (C_ij - conj(C_ji)).  X is
 // double-buffered: the pass reads X[cur] and writes X[cur ^ 1].
 template <typename R>
-__host__ __device__ __forceinline__ ResLayout<R> res_layout_direct(int n, int M, int P, int nt_ept, bool comp = false)
+__host__ __device__ __forceinline__ ResLayout<R> res_layout_direct(int n, int M, int P, int nt_ept, bool comp = false,
+                                                                   bool dense_coul = false)
 {
     ResLayout<R> L;
     const size_t RP = (size_t)((M * n) | 1);
@@ -514,9 +787,10 @@ __host__ __device__ __forceinline__ ResLayout<R> res_layout_direct(int n, int M,
     L.rho = o;  o = align16(o + sizeof(cplx<R>) * (size_t)nt_ept);
     L.dd = o;   o = align16(o + sizeof(R) * 2 * (size_t)M * n);   // double-buffered
     L.dg = o;   o = align16(o + sizeof(R) * 2 * ((size_t)M * n + 1));
-    L.es = o;   o = align16(o + sizeof(double) * 4 * ((size_t)M + 32));   // per matrix, then per warp
+    L.es = o;   o = align16(o + sizeof(double) * 4 * 32);               // energy partials per warp
     L.ell = o;  o = align16(o + sizeof(Ent<R>) * (size_t)n * (2 * P + 1));
     L.lo = o;   if (comp) o = align16(o + sizeof(uint32_t) * (size_t)nt_ept);   // bf16 residual pairs
+    L.xs = o;   if (dense_coul) o = align16(o + sizeof(R) * coul_scratch<R>(M * n));
     L.total = o;
     return L;
 }
@@ -538,12 +812,14 @@ __device__ __forceinline__ void res_direct_pass(const cplx<R>* __restrict__ X, c
                                                 R h, int tid, int n, int RP, int spare, int dgspare,
                                                 cplx<R>* __restrict__ dump_in, cplx<R>* __restrict__ dump_out,
                                                 const DumpMap dm, const DdNext dnx, const DevSys<R>& sys,
-                                                const R* __restrict__ udiag, R pvn, uint32_t* __restrict__ loS)
+                                                const R* __restrict__ udiag, R pvn, uint32_t* __restrict__ loS,
+                                                int E)
 {
     constexpr int NE = 2 * P + 1;
 #pragma unroll
     for (int q = 0; q < EPT; ++q) {
         const int f = tid + q * NT;
+        if ((tid & ~31) + q * NT >= E) break;               // this warp's remaining slots are empty
         const bool valid = ix[q] != ~0u;
         const int i = valid ? (int)(ix[q] & 1023u) : 0;
         const int j = valid ? (int)((ix[q] >> 10) & 1023u) : 0;
@@ -672,7 +948,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(ResArgs<R> a)
     const int SPARE = n * RP;
     constexpr int NE = 2 * P + 1;
     const bool comp = std::is_same<R, float>::value && a.state64 != nullptr;
-    const ResLayout<R> L = res_layout_direct<R>(n, M, P, NT * EPT, comp);
+    const ResLayout<R> L = res_layout_direct<R>(n, M, P, NT * EPT, comp, a.sys.ud != nullptr);
     uint32_t* loS = comp ? reinterpret_cast<uint32_t*>(smem + L.lo) : nullptr;
     cplx<R>* Xb = reinterpret_cast<cplx<R>*>(smem + L.x);
     cplx<R>* rhoS = reinterpret_cast<cplx<R>*>(smem + L.rho);
@@ -774,58 +1050,8 @@ __global__ void __launch_bounds__(NT, 1) k_resident(ResArgs<R> a)
         bar();
         for (int t = a.t_begin; t < a.t_end; ++t) {
             if (a.record) {
-                const cplx<R>* X = Xb + cur * XS;
-                const R* d0 = dg + cur * DGS;
-                const int nvec = SPLIT ? (rank == 0 ? 3 : 2) : 5;
-                for (int w = tid; w < nvec * n; w += NT) {
-                    const int oo = w / n, j = w - oo * n;
-                    int o;
-                    if (SPLIT) o = rank == 0 ? (oo == 0 ? 0 : oo == 1 ? 2 : 4) : (oo == 0 ? 1 : 3);
-                    else o = oo;
-                    double acc = 0.0;
-                    for (int g = 0; g < a.G; ++g) {
-                        if (gid * a.G + g >= a.B) break;
-                        double du, dd;
-                        if (SPLIT) {
-                            const double mine = (double)d0[g * n + j], oth = (double)other_dg(cur, g)[j];
-                            du = rank == 0 ? mine : oth;
-                            dd = rank == 0 ? oth : mine;
-                        } else {
-                            du = (double)d0[(2 * g) * n + j];
-                            dd = (double)d0[(2 * g + 1) * n + j];
-                        }
-                        if (!isfinite(du) || !isfinite(dd)) atomicOr(a.err, 1u);
-                        acc += o == 0 ? du : o == 1 ? dd : o == 2 ? du * du : o == 3 ? dd * dd : du * dd;
-                    }
-                    atomicAdd(myslot + (size_t)t * W + o * n + j, acc);
-                }
-                if (a.do_en) {
-                    // every thread of the CTA works on each matrix in turn
-                    double* ew = es + 4 * M;              // per-warp partials
-                    for (int m = 0; m < M; ++m) {
-                        const int g = SPLIT ? m : (m >> 1), s = SPLIT ? rank : (m & 1);
-                        double e[4] = {0.0, 0.0, 0.0, 0.0};
-                        energy_partials_full<R>(a.sys, X, RP, m * n, d0 + m * n, other_dg(cur, m), s, a.do_e1,
-                                                a.do_e2, tid, NT, e);
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            const double v = warp_sum(e[c]);
-                            if (lane == 0) ew[warp * 4 + c] = v;
-                        }
-                        __syncthreads();
-                        if (tid < 4) {
-                            double v = 0.0;
-                            for (int q = 0; q < NW; ++q) v += ew[q * 4 + tid];
-                            es[m * 4 + tid] = (gid * a.G + g < a.B) ? v : 0.0;
-                        }
-                        __syncthreads();
-                    }
-                    if (tid < 4) {
-                        double acc = 0.0;
-                        for (int m = 0; m < M; ++m) acc += es[m * 4 + tid];
-                        atomicAdd(myslot + (size_t)t * W + 5 * n + tid, acc);
-                    }
-                }
+                res_record<R, NT, SPLIT>(a, [&](int m, int k, int j) { return Xb[cur * XS + j * RP + m * n + k].re; },
+                                         dg + cur * DGS, [&](int m) { return other_dg(cur, m); }, es, myslot + (size_t)t * W, gid, rank, tid);
                 if (a.whole) {
 #pragma unroll
                     for (int q = 0; q < EPT; ++q) {
@@ -847,11 +1073,9 @@ __global__ void __launch_bounds__(NT, 1) k_resident(ResArgs<R> a)
                     R* Dc = Dd + dcur * RR;
                     if (!dd_ok) {
                         const R pv = a.sys.n_bins > 0 ? a.ptab[(gstep - a.step_base) * 4 + stage] : R(0);
-                        for (int w = tid; w < RR; w += NT) {
-                            const int m = w / n, j = w - m * n;
-                            Dc[w] = delta_diag_v<R>(a.sys, j, dg + cur * DGS + m * n, other_dg(cur, m), pv);
-                        }
-                        __syncthreads();
+                        delta_diag_block<R, NT, !SPLIT>(a.sys, a.sys.ud, a.sys.vd, Dc, reinterpret_cast<R*>(smem + L.xs), RR,
+                                                [&](int m) { return dg + cur * DGS + m * n; },
+                                                [&](int m) { return other_dg(cur, m); }, pv, tid);
                     }
                     // does another stage follow in this launch (possibly after a record)?
                     const bool more = stage < 3 || st + 1 < nsteps ||
@@ -872,10 +1096,10 @@ __global__ void __launch_bounds__(NT, 1) k_resident(ResArgs<R> a)
                         dout = din + (size_t)(stage + 1) * a.dump_count;
                     }
                     const DumpMap dm = {gid * a.G, rank, a.B, ne, SPLIT ? 1 : 0};
-                    if (stage == 0) res_direct_pass<R, NT, EPT, 0, P, DUMP>(X, Xn, ell, Dc, rhoS, dgn, ix, Ar, Br, a.h, tid, n, RP, SPARE, RR, din, dout, dm, dnx, a.sys, a.udiag, pvn, loS);
-                    else if (stage == 1) res_direct_pass<R, NT, EPT, 1, P, DUMP>(X, Xn, ell, Dc, rhoS, dgn, ix, Ar, Br, a.h, tid, n, RP, SPARE, RR, din, dout, dm, dnx, a.sys, a.udiag, pvn, loS);
-                    else if (stage == 2) res_direct_pass<R, NT, EPT, 2, P, DUMP>(X, Xn, ell, Dc, rhoS, dgn, ix, Ar, Br, a.h, tid, n, RP, SPARE, RR, din, dout, dm, dnx, a.sys, a.udiag, pvn, loS);
-                    else res_direct_pass<R, NT, EPT, 3, P, DUMP>(X, Xn, ell, Dc, rhoS, dgn, ix, Ar, Br, a.h, tid, n, RP, SPARE, RR, din, dout, dm, dnx, a.sys, a.udiag, pvn, loS);
+                    if (stage == 0) res_direct_pass<R, NT, EPT, 0, P, DUMP>(X, Xn, ell, Dc, rhoS, dgn, ix, Ar, Br, a.h, tid, n, RP, SPARE, RR, din, dout, dm, dnx, a.sys, a.udiag, pvn, loS, E);
+                    else if (stage == 1) res_direct_pass<R, NT, EPT, 1, P, DUMP>(X, Xn, ell, Dc, rhoS, dgn, ix, Ar, Br, a.h, tid, n, RP, SPARE, RR, din, dout, dm, dnx, a.sys, a.udiag, pvn, loS, E);
+                    else if (stage == 2) res_direct_pass<R, NT, EPT, 2, P, DUMP>(X, Xn, ell, Dc, rhoS, dgn, ix, Ar, Br, a.h, tid, n, RP, SPARE, RR, din, dout, dm, dnx, a.sys, a.udiag, pvn, loS, E);
+                    else res_direct_pass<R, NT, EPT, 3, P, DUMP>(X, Xn, ell, Dc, rhoS, dgn, ix, Ar, Br, a.h, tid, n, RP, SPARE, RR, din, dout, dm, dnx, a.sys, a.udiag, pvn, loS, E);
                     bar();
                     cur ^= 1;
                     dcur ^= 1;

@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "fpsg_kernels.cuh"
+#include "fpsg_pair.cuh"
 #include "fpsg_quad.cuh"
 
 namespace fpsg {
@@ -27,6 +28,15 @@ template <>
 const std::vector<ResCfg<float>>& res_cfgs<float>();
 template <>
 const std::vector<ResCfg<double>>& res_cfgs<double>();
+
+// configurations of k_pair; ept counts slots per thread, fn[] is for 2 and 3 offsets
+template <typename R>
+const std::vector<ResCfg<R>>& pair_cfgs();
+
+template <>
+const std::vector<ResCfg<float>>& pair_cfgs<float>();
+template <>
+const std::vector<ResCfg<double>>& pair_cfgs<double>();
 
 // 4-CTA-cluster configurations (k_resident_quad): two CTAs per spin matrix
 template <typename R>
@@ -64,6 +74,9 @@ const std::vector<QuadCfg<double>>& quad_hp_cfgs<double>();
      {k_resident<R, NT, EPT, SPLIT, 2>, k_resident<R, NT, EPT, SPLIT, 4>, k_resident<R, NT, EPT, SPLIT, 8>}, \
      {k_resident<R, NT, EPT, SPLIT, 2, true>, k_resident<R, NT, EPT, SPLIT, 4, true>,                     \
       k_resident<R, NT, EPT, SPLIT, 8, true>}}
+#define FPSG_PAIR(R, NT, SPT, SPLIT)                                                  \
+    {NT, SPT, SPLIT, {k_pair<R, NT, SPT, SPLIT, 2>, k_pair<R, NT, SPT, SPLIT, 3>},  \
+     {k_pair<R, NT, SPT, SPLIT, 2, true>, k_pair<R, NT, SPT, SPLIT, 3, true>}}
 
 #define FPSG_QUAD(R, NT, EPT)                                                                     \
     {NT, EPT, {k_resident_quad<R, NT, EPT, 5>, k_resident_quad<R, NT, EPT, 9>, k_resident_quad<R, NT, EPT, 13>, \

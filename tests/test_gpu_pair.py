@@ -1,0 +1,74 @@
+"""k_pair (offset-pattern lattices) against the oracle, at the sizes where its slot order,
+masks and dispatch change: tiles of 32 rows and their remainders, odd and even n, one, two
+and three offsets, sites without neighbours, one matrix per CTA and many, split and not."""
+import numpy as np
+import pytest
+
+from fermiphasespace_b200 import configs as cf
+from fermiphasespace_b200 import engine as E
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def lattice(nx, ny, nz, t):
+    return cf.hopping(cf.distances(cf.grid_positions(nx, ny, nz)), [(1.0, t)] if t else [])
+
+
+def compare(T, coulomb, ext, B, S=2, Tp=4, dt=0.01, seed=3):
+    n = T.shape[0]
+    rng = np.random.default_rng(seed)
+    if coulomb == E.COUL_DISTANCE:
+        D = np.abs(np.arange(n)[:, None] - np.arange(n)[None, :])
+        U = 2.0 / (1.0 + D)
+        V = U - np.diag(np.diag(U))
+    else:
+        U, V = np.diag(rng.uniform(1.0, 4.0, n)), None
+    X = np.diag(rng.uniform(-1, 1, n)) if ext else None
+    occ = (rng.random(n) < 0.5).astype(float)
+    rho = orc.sample(n, B, 11, occ, 1.0 - occ)
+    ref = orc.run(orc.System(T, U, V, X, coulomb, X is None), 0, dt, S, Tp, rho)
+    out = {}
+    for prec in (E.PREC_FP64, E.PREC_FP32):
+        eng = E.Engine()
+        eng.set_system(T, U, V, X, coulomb)
+        eng.set_initial_samples(rho)
+        r = eng.run(E.METHOD_FTWA, prec, dt, S, Tp)
+        assert r.path_used == E.PATH_RESIDENT
+        out[prec] = (r, eng.get_state())
+        eng.close()
+    return ref, out
+
+
+@pytest.mark.parametrize("dims,t,coulomb,ext,B", [
+    ((1, 1, 1), 0.0, E.COUL_ONSITE, False, 5),      # one site, no offsets
+    ((2, 1, 1), -1.0, E.COUL_ONSITE, True, 40),
+    ((7, 1, 1), -0.7, E.COUL_ONSITE, False, 300),   # a chain: one offset, several matrices per CTA
+    ((31, 1, 1), -1.0, E.COUL_DISTANCE, True, 3),   # one partial tile
+    ((8, 4, 1), -1.3, E.COUL_ONSITE, True, 3),      # exactly one tile of 32
+    ((11, 3, 1), -1.0, E.COUL_ONSITE, False, 3),    # a tile and one row
+    ((7, 9, 1), -1.0, E.COUL_DISTANCE, False, 3),   # 63: odd last column beside a full tile
+    ((8, 8, 1), 0.9, E.COUL_ONSITE, True, 4),       # 64: two tiles
+    ((4, 4, 4), -1.0, E.COUL_ONSITE, False, 3),     # three offsets
+    ((3, 4, 5), -0.3, E.COUL_DISTANCE, True, 3),
+    ((3, 9, 3), -1.0, E.COUL_ONSITE, True, 2),      # 81, three offsets
+])
+def test_pair_matches_oracle(dims, t, coulomb, ext, B):
+    ref, out = compare(lattice(*dims, t), coulomb, ext, B)
+    r, state = out[E.PREC_FP64]
+    assert np.array_equal(state, ref["final"])
+    for k in ("niiu", "niid", "n2iiu", "n2iid", "nund", "energies"):
+        assert np.allclose(getattr(r, k), ref[k], rtol=1e-13, atol=1e-13), k
+    # FP32: 8 steps of 4 stages round |rho| <= 2 (samples included) to 2^-24 a few times each, the
+    # update itself compensated: h |Delta| <= 0.2 of a few ulp per stage
+    r, state = out[E.PREC_FP32]
+    assert np.max(np.abs(state - ref["final"])) < 32 * 0.2 * 8 * 2.0 * 2.0 ** -24 * 4
+
+
+def test_pattern_needs_one_value():
+    """Hopping of two values has no offset pattern: the column kernels run it, to the same bits."""
+    T = cf.hopping(cf.distances(cf.grid_positions(5, 4)), [(1.0, -1.0)])
+    T[0, 1] = T[1, 0] = -1.5
+    ref, out = compare(T, E.COUL_ONSITE, True, 3)
+    assert np.array_equal(out[E.PREC_FP64][1], ref["final"])
+
