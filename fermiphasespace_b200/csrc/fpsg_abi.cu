@@ -639,6 +639,25 @@ ResPlan plan_quad(fpsg_ctx* ctx, bool comp)
     return best;
 }
 
+// k_pair_packed for a Delta with an offset pattern, where k_pair does not fit.
+template <typename R>
+ResPlan plan_packed(fpsg_ctx* ctx, bool comp)
+{
+    ResPlan best;
+    const DevTables<R>& t = tables<R>(ctx);
+    if (t.pat_ns == 0 || ctx->n > PAIR_NMAX) return best;
+    const auto& cf = packed_cfgs<R>();
+    for (int c = 0; c < (int)cf.size(); ++c) {
+        const int cap = cf[c].nt * cf[c].ept;
+        if (cap < ctx->n_pair) continue;
+        const size_t sm = packed_layout<R>(ctx->n, cap, comp, t.pat.off[0], t.ud != nullptr).total;
+        if (sm > ctx->smem_optin) continue;
+        best.idx = c; best.G = 1; best.smem = sm; best.quad = best.pair = true; best.comp = comp; best.nh = 1;
+        break;
+    }
+    return best;
+}
+
 // The resident configuration of a run: one CTA (or 2-CTA cluster) per matrix group
 // when it fits, else two CTAs per spin; FP32 with the compensated state update when
 // its residuals fit too (and the context does not ask for the plain update).
@@ -649,6 +668,17 @@ ResPlan choose_resident(fpsg_ctx* ctx, int B)
     ResPlan plan;
     if (comp_ok) plan = plan_resident<R>(ctx, B, true);
     if (plan.idx < 0) plan = plan_resident<R>(ctx, B);
+    if (plan.idx < 0 || !plan.pair) {
+        const ResPlan pk = plan_packed<R>(ctx, comp_ok);
+        if (pk.idx >= 0) plan = pk;
+        // few trajectories: one wave of 4-CTA clusters (four SMs per trajectory) ends before
+        // one of 2-CTA clusters does (10x10 grid, FP64, 1 trajectory x 400 steps: 10.3 against
+        // 13.0 ms), but only a quarter of the SM count of them run at a time
+        if (std::is_same<R, double>::value && pk.idx >= 0 && B <= ctx->sm_count / 5) {
+            const ResPlan two = plan_quad<R>(ctx, false);
+            if (two.idx >= 0 && two.hp) plan = two;
+        }
+    }
     if (plan.idx < 0 && comp_ok) plan = plan_quad<R>(ctx, true);
     if (plan.idx < 0) plan = plan_quad<R>(ctx, false);
     return plan;
@@ -695,9 +725,9 @@ struct ResLauncher {
     {
         if (plan.quad) {
             if (dump) return fail(ctx, FPSG_ERR_UNSUPPORTED, "the 4-CTA resident kernel keeps no stage inputs");
-            const QuadCfg<R>& qc = plan.hp ? quad_hp_cfgs<R>()[plan.idx] : quad_cfgs<R>()[plan.idx];
-            fn = (plan.hp && plan.e8 ? qc.fn8 : qc.fn)[quad_w_index(tables<R>(ctx).cell_w)];
-            nt = qc.nt; split = false; cdim = plan.hp ? 2 * plan.nh : 4; smem = plan.smem;
+            const QuadCfg<R>& qc = (plan.pair ? packed_cfgs<R>() : plan.hp ? quad_hp_cfgs<R>() : quad_cfgs<R>())[plan.idx];
+            fn = (plan.hp && plan.e8 ? qc.fn8 : qc.fn)[plan.pair ? tables<R>(ctx).pat_ns - 2 : quad_w_index(tables<R>(ctx).cell_w)];
+            nt = qc.nt; split = false; cdim = plan.hp || plan.pair ? 2 * plan.nh : 4; smem = plan.smem;
             CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             cudaLaunchConfig_t lc = config(ctx, cdim * B);
             cudaLaunchAttribute at[1];

@@ -1,0 +1,15 @@
+// fpsg_packed_f32.cu — FP32 configurations of k_pair_packed.
+#include "fpsg_resident.h"
+
+namespace fpsg {
+
+template <>
+const std::vector<QuadCfg<float>>& packed_cfgs<float>()
+{
+    static const std::vector<QuadCfg<float>> v = {
+        FPSG_PACKED(float, 512, 6), FPSG_PACKED(float, 512, 8),
+    };
+    return v;
+}
+
+}  // namespace fpsg

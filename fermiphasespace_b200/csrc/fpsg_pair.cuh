@@ -587,4 +587,329 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_pair(ResArgs<R> a)
     }
 }
 
+// ------------------------------------------------------------------------------
+// k_pair_packed — the pair kernel for one spin matrix per CTA that does not fit twice.
+//
+// The terms of an upper element reach at most D = off[0] rows below the diagonal, so X is
+// kept once, as the upper triangle and the D sub-diagonals, column j in j + D + 1 entries:
+//     X(r, c) at C(c) + r,   C(c) = c (c + 2 D + 1) / 2,
+// about half of the full matrix, with C(j + o) - C(j) linear in j.  With the state beside it
+// that is 194 KB in FP64 at n = 100: a spin on ONE CTA, where k_resident_quad_hp takes two
+// (33 four-CTA clusters on 132 SMs; every new element crosses to the sibling through
+// distributed shared memory, 16 bytes a cycle; a 460-cycle cluster barrier per stage).  X is
+// single-buffered: a pass computes k of every slot into the RK registers, and after a block
+// barrier (45 cycles) a second one forms the new stage input from the registers and the
+// state and stores it, so no stage output is held across the barrier.  FP64 keeps k1 and k2
+// themselves and forms A = k1 - k2 and Bc = k1 + 3 k2 one stage later, by the same
+// operations: bit-identical to the oracle.
+// 10x10 grid, FP64, 4096 trajectories x 41 steps: 134.7 -> 77.0 ms
+__host__ __device__ __forceinline__ int packed_col(int c, int D) { return (c * (c + 2 * D + 1)) >> 1; }
+
+template <int NS>
+struct PackedAddr {
+    int j, D;
+    const int (&off)[PAT_MAX];
+    __device__ __forceinline__ int next() const { return j + D + 1; }
+    // C(j + e + sgn off) - C(j), from C(c + o) - C(c) = o c + o (o + 2 D + 1) / 2
+    __device__ __forceinline__ int col(int s, int sgn, int e) const
+    {
+        const int o = s == NS - 1 ? 1 : off[s];
+        const int d = sgn * o + e;
+        return d * j + ((d * (d + 2 * D + 1)) >> 1);
+    }
+};
+
+template <typename R>
+__host__ __device__ __forceinline__ ResLayout<R> packed_layout(int n, int slots, bool comp, int D, bool dense_coul)
+{
+    ResLayout<R> L;
+    // masked neighbours: C(c) >= -D (D + 1) / 2 for c >= -D, and columns up to n + D
+    const size_t before = sizeof(cplx<R>) * (size_t)(D * (D + 1) / 2 + D + 1);
+    const size_t after = sizeof(cplx<R>) * (size_t)(packed_col(n + D + 1, D) + n - packed_col(n, D));
+    size_t o = 0;
+    L.dd = o;   o = align16(o + sizeof(R) * 6 * ((size_t)n + 1));
+    L.dg = o;   o = align16(o + sizeof(R) * 2 * ((size_t)n + 1));
+    L.sd = o;   o = align16(o + sizeof(R) * 4 * (size_t)n + 32);
+    L.es = o;   o = align16(o + sizeof(double) * 4 * 32);
+    L.xs = o;   if (dense_coul) o = align16(o + sizeof(R) * coul_scratch<R>(n));
+    if (o < before) o = align16(before);
+    L.x = o;    o = align16(o + sizeof(cplx<R>) * (size_t)packed_col(n, D));
+    const size_t x_end = o;
+    L.rho = o;  o = align16(o + sizeof(cplx<R>) * 2 * (size_t)slots);
+    L.lo = o;   if (comp) o = align16(o + sizeof(uint32_t) * 2 * (size_t)slots);
+    if (o < x_end + after) o = align16(x_end + after);
+    L.ell = L.uv = o;
+    L.total = o;
+    return L;
+}
+
+// FP64 stage inputs and accumulators (see rk_update): a, b hold k1, k2 up to stage 3, then
+// A + k3 and Bc + 3 k3
+__device__ __forceinline__ void packed_acc(int stage, double k, double& a, double& b)
+{
+    if (stage == 0) { a = k; return; }
+    if (stage == 1) { b = k; return; }
+    if (stage == 2) {
+        const double A = __dsub_rn(a, b), Bc = __dadd_rn(a, __dmul_rn(b, 3.0));
+        a = __dadd_rn(A, k);
+        b = __dadd_rn(Bc, __dmul_rn(k, 3.0));
+        return;
+    }
+    a = k;
+}
+__device__ __forceinline__ double packed_next(int stage, double rho, double a, double b, double h)
+{
+    if (stage == 0) return __dadd_rn(rho, div3_rn(__dmul_rn(a, h)));
+    if (stage == 1) return __dadd_rn(rho, __dmul_rn(__dadd_rn(div3_rn(-a), b), h));
+    if (stage == 2) return __dadd_rn(rho, __dmul_rn(a, h));
+    return __dadd_rn(rho, __dmul_rn(__dmul_rn(__dadd_rn(b, a), h), 0.125));
+}
+
+template <typename R, int NT, int SPT, int NS>
+__global__ void __launch_bounds__(NT, 1) k_pair_packed(ResArgs<R> a)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr bool kFloat = std::is_same<R, float>::value;
+    const int n = a.sys.n, ne = a.sys.ne, D = a.pat.off[0];
+    const int E = a.nslots, DS = n + 1;
+    const bool comp = kFloat && a.state64 != nullptr;
+    const ResLayout<R> L = packed_layout<R>(n, NT * SPT, comp, D, a.sys.ud != nullptr);
+    cplx<R>* X = reinterpret_cast<cplx<R>*>(smem + L.x);
+    cplx<R>* rhoS = reinterpret_cast<cplx<R>*>(smem + L.rho);
+    uint32_t* loS = reinterpret_cast<uint32_t*>(smem + L.lo);
+    R* Dd = reinterpret_cast<R*>(smem + L.dd);      // [3][DS], and the other spin's diagonal [3][DS]
+    R* od = Dd + 3 * DS;
+    R* dg = reinterpret_cast<R*>(smem + L.dg);
+    R* sd = reinterpret_cast<R*>(smem + L.sd);
+    double* es = reinterpret_cast<double*>(smem + L.es);
+    R* scr = reinterpret_cast<R*>(smem + L.xs);
+    const int tid = threadIdx.x;
+    const int W = rec_width(n);
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank();
+    const int cid = blockIdx.x >> 1, ncl = gridDim.x >> 1;
+    // the exchange of diagonals with the other spin's CTA is k_pair's
+    const uint32_t mbar_a = (uint32_t)__cvta_generic_to_shared(smem + L.sd + align16(sizeof(R) * 4 * (size_t)n));
+    const uint32_t p_dd = peer_addr(Dd, rank ^ 1), p_od = peer_addr(od, rank ^ 1), p_bar = peer_addr(smem + L.sd + align16(sizeof(R) * 4 * (size_t)n), rank ^ 1);
+    if (tid < 3) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar_a + 8 * tid) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    uint32_t ph = 0, parity = 0;
+    bool lost = false;
+
+    typename PairAcc<R>::T Ar[2 * SPT], Br[2 * SPT];
+    uint32_t ix[SPT], fl[SPT];
+#pragma unroll
+    for (int q = 0; q < SPT; ++q) {
+        const int f = tid + q * NT;
+        ix[q] = 0u;
+        fl[q] = PAIR_NONE | PAIR_ONE;
+        const uint32_t p = f < E ? a.order[f] : ~0u;
+        if (p == ~0u) continue;
+        const uint32_t i = p & 0xffffu, j = (p >> 16) & 0x7fffu;
+        const bool one = (p & PAIR_NONE) != 0;
+        ix[q] = i | (j << 10);
+        fl[q] = a.pat.mask[j] | ((one ? 0u : a.pat.mask[j + 1]) << (2 * NS)) | (a.pat.mask[i] << (4 * NS)) |
+                (one ? PAIR_ONE : 0u);
+    }
+    auto i_of = [&](int q) { return (int)(ix[q] & 1023u); };
+    auto j_of = [&](int q) { return (int)(ix[q] >> 10); };
+    for (int q = tid; q < 6 * DS; q += NT) Dd[q] = R(0);
+    for (int j = tid; j < n; j += NT) {
+        sd[j] = a.sys.tdiag[j];
+        sd[n + j] = a.udiag ? a.udiag[j] : R(0);
+        sd[2 * n + j] = a.sys.ediag[j];
+        sd[3 * n + j] = a.sys.proj[j];
+    }
+    for (int q = tid; q < packed_col(n, D); q += NT) X[q] = cplx<R>{R(0), R(0)};   // rows past n - 1
+    double* myslot = a.slots ? a.slots + (size_t)blockIdx.x * a.Tp * W : nullptr;
+    cl.sync();
+    for (int b = cid; b < a.B; b += ncl) {
+        const size_t base = ((size_t)b * 2 + rank) * ne;
+#pragma unroll
+        for (int q = 0; q < SPT; ++q) {
+            const int f = tid + q * NT, i = i_of(q), j = j_of(q);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                cplx<R> v = {R(0), R(0)};
+                uint32_t lo = 0;
+                if (!(fl[q] & PAIR_NONE) && !(e && (fl[q] & PAIR_ONE))) {
+                    const int c = j + e;
+                    if (comp) {
+                        const cplx<double> x = a.state64[base + cs(c) + i];
+                        v.re = (R)x.re;
+                        v.im = (R)x.im;
+                        lo = pack_bf16x2((float)(x.re - (double)v.re), (float)(x.im - (double)v.im));
+                    } else {
+                        v = a.state[base + cs(c) + i];
+                    }
+                    if (c - i <= D) X[packed_col(i, D) + c] = cplx<R>{v.re, -v.im};
+                    X[packed_col(c, D) + i] = v;
+                    if (i == c) {
+                        dg[i] = v.re;
+                        st_peer(p_od + (uint32_t)((ph * DS + i) * (int)sizeof(R)), v.re);
+                    }
+                }
+                rhoS[2 * f + e] = v;
+                if (comp) loS[2 * f + e] = lo;
+                Ar[2 * q + e] = Br[2 * q + e] = {};
+            }
+        }
+        bool dd_ok = false;                  // Dd[ph] already holds this stage's diagonal
+        long gstep = a.step_base;
+        cl.sync();
+        for (int t = a.t_begin; t < a.t_end; ++t) {
+            if (a.record) {
+                res_record<R, NT, true>(a, [&](int, int k, int j) { return X[packed_col(j, D) + k].re; }, dg,
+                                        [&](int) { return od + ph * DS; }, es, myslot + (size_t)t * W, b, rank, tid);
+                if (a.whole) {
+#pragma unroll
+                    for (int q = 0; q < SPT; ++q) {
+                        if (fl[q] & PAIR_NONE) continue;
+                        const int f = tid + q * NT, i = i_of(q), j = j_of(q);
+                        double2* w = a.whole + ((size_t)t * 2 + rank) * ne;
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            if (e && (fl[q] & PAIR_ONE)) continue;
+                            atomicAdd(&w[cs(j + e) + i].x, (double)rhoS[2 * f + e].re);
+                            atomicAdd(&w[cs(j + e) + i].y, (double)rhoS[2 * f + e].im);
+                        }
+                    }
+                }
+            }
+            const int nsteps = (a.hf && t == a.Tp - 1) ? 0 : a.S;
+            for (int st = 0; st < nsteps; ++st, ++gstep) {
+#pragma unroll 1
+                for (int stage = 0; stage < 4; ++stage) {
+                    R* Dc = Dd + ph * DS;
+                    if (!dd_ok) {
+                        const R pv = a.sys.n_bins > 0 ? a.ptab[(gstep - a.step_base) * 4 + stage] : R(0);
+                        delta_diag_block<R, NT, false>(a.sys, a.sys.ud, a.sys.vd, Dc, scr, n, [&](int) { return dg; },
+                                                       [&](int) { return od + ph * DS; }, pv, tid);
+                    }
+                    const bool more = stage < 3 || st + 1 < nsteps ||
+                                      (t + 1 < a.t_end && a.S > 0 && !(a.hf && t + 1 == a.Tp - 1));
+                    const bool fuse = a.udiag != nullptr && more;
+                    const R pvn = fuse && a.sys.n_bins > 0 ? a.ptab[(gstep - a.step_base) * 4 + stage + 1] : R(0);
+                    const uint32_t nph = ph == 2 ? 0 : ph + 1;
+                    if (tid == 0)
+                        asm volatile("{\n\t.reg .b64 s;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 s, [%0], %1;\n\t}"
+                                     ::"r"(mbar_a + 8 * nph), "r"((uint32_t)(2 * n * (int)sizeof(R))) : "memory");
+                    // k of every slot
+#pragma unroll
+                    for (int q = 0; q < SPT; ++q) {
+                        if ((tid & ~31) + q * NT >= E) break;       // this warp's remaining slots are empty
+                        const int i = i_of(q), j = j_of(q);
+                        const PackedAddr<NS> ad = {j, D, a.pat.off};
+                        const int xo = packed_col(j, D) + i;
+                        if constexpr (kFloat) {
+                            const uint64_t* xp = reinterpret_cast<const uint64_t*>(X) + xo;
+                            const uint64_t o0 = xp[0], o1 = xp[ad.next()];
+                            uint64_t g0, g1;
+                            pair_sums_f32<NS>(xp, ad, fl[q], a.pat, o0, o1, Dc[i], Dc[j], Dc[j + 1], g0, g1);
+                            if (stage == 0) { Ar[2 * q] = g0; Ar[2 * q + 1] = g1; }
+                            else if (stage == 1) { Br[2 * q] = g0; Br[2 * q + 1] = g1; }
+                            else if (stage == 2) {
+                                f2_stage(2, 0, g0, Ar[2 * q], Br[2 * q], a.h);
+                                f2_stage(2, 0, g1, Ar[2 * q + 1], Br[2 * q + 1], a.h);
+                            } else { Ar[2 * q] = g0; Ar[2 * q + 1] = g1; }
+                        } else {
+                            cplx<R> k0, k1;
+                            pair_sums_f64<NS>(X + xo, ad, fl[q], a.pat, Dc[i], Dc[j], Dc[j + 1], k0, k1);
+                            packed_acc(stage, k0.re, Ar[2 * q].re, Br[2 * q].re);
+                            packed_acc(stage, k0.im, Ar[2 * q].im, Br[2 * q].im);
+                            packed_acc(stage, k1.re, Ar[2 * q + 1].re, Br[2 * q + 1].re);
+                            packed_acc(stage, k1.im, Ar[2 * q + 1].im, Br[2 * q + 1].im);
+                        }
+                    }
+                    __syncthreads();         // every thread is done reading X
+#pragma unroll
+                    for (int q = 0; q < SPT; ++q) {
+                        const int f = tid + q * NT;
+                        if ((tid & ~31) + q * NT >= E) break;
+                        const int i = i_of(q), j = j_of(q);
+                        cplx<R> x0, x1;
+                        if constexpr (kFloat) {
+                            const ulonglong2 rr = reinterpret_cast<const ulonglong2*>(rhoS)[f];
+                            ulonglong2 y;
+                            if (stage < 3) {
+                                y.x = f2_stage_input(stage + 1, rr.x, Ar[2 * q], Br[2 * q], a.h);
+                                y.y = f2_stage_input(stage + 1, rr.y, Ar[2 * q + 1], Br[2 * q + 1], a.h);
+                            } else {
+                                uint2 lo = make_uint2(0u, 0u);
+                                if (comp) lo = reinterpret_cast<const uint2*>(loS)[f];
+                                y.x = f2_final(rr.x, Ar[2 * q], Br[2 * q], a.h, comp, lo.x);
+                                y.y = f2_final(rr.y, Ar[2 * q + 1], Br[2 * q + 1], a.h, comp, lo.y);
+                                if (comp) reinterpret_cast<uint2*>(loS)[f] = lo;
+                                reinterpret_cast<ulonglong2*>(rhoS)[f] = y;
+                            }
+                            x0 = f2_unpack(y.x);
+                            x1 = f2_unpack(y.y);
+                        } else {
+                            const cplx<R> r0 = rhoS[2 * f], r1 = rhoS[2 * f + 1];
+                            x0.re = packed_next(stage, r0.re, Ar[2 * q].re, Br[2 * q].re, a.h);
+                            x0.im = packed_next(stage, r0.im, Ar[2 * q].im, Br[2 * q].im, a.h);
+                            x1.re = packed_next(stage, r1.re, Ar[2 * q + 1].re, Br[2 * q + 1].re, a.h);
+                            x1.im = packed_next(stage, r1.im, Ar[2 * q + 1].im, Br[2 * q + 1].im, a.h);
+                            if (stage == 3) { rhoS[2 * f] = x0; rhoS[2 * f + 1] = x1; }
+                        }
+                        if (fl[q] & PAIR_NONE) continue;
+                        const int cj = packed_col(j, D), ci = packed_col(i, D);
+                        if (j - i <= D) X[ci + j] = cplx<R>{x0.re, -x0.im};
+                        X[cj + i] = x0;                       // on the diagonal this second store wins
+                        if (!(fl[q] & PAIR_ONE)) {
+                            if (j + 1 - i <= D) X[ci + j + 1] = cplx<R>{x1.re, -x1.im};
+                            X[cj + j + D + 1 + i] = x1;
+                        }
+                        if (i == j) {
+                            dg[i] = x0.re;
+                            R d = R(0);
+                            if (fuse) {
+                                // Delta_ii of the other spin for the next stage (on-site U only)
+                                d = sd[i];
+                                if (a.sys.coul != 0) {
+                                    R u = R(0);
+                                    const R uu = sd[n + i];
+                                    if (uu != R(0)) u = fmaR<R>(uu, addR<R>(x0.re, a.sys.shift), u);
+                                    d = addR<R>(d, u);
+                                }
+                                if (a.sys.has_ext) d = addR<R>(d, sd[2 * n + i]);
+                                if (a.sys.n_bins > 0) d = addR<R>(d, mulR<R>(pvn, sd[3 * n + i]));
+                            }
+                            const uint32_t o = (nph * DS + i) * (uint32_t)sizeof(R);
+                            st_async(p_dd + o, d, p_bar + 8 * nph);
+                            st_async(p_od + o, x0.re, p_bar + 8 * nph);
+                        }
+                    }
+                    __syncthreads();
+                    if (!lost && !peer_wait(mbar_a + 8 * nph, (parity >> nph) & 1u)) {
+                        lost = true;
+                        atomicOr(a.err, ERR_PEER_WAIT);
+                    }
+                    parity ^= 1u << nph;
+                    ph = nph;
+                    dd_ok = fuse;
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < SPT; ++q) {
+            if (fl[q] & PAIR_NONE) continue;
+            const int f = tid + q * NT, i = i_of(q), j = j_of(q);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                if (e && (fl[q] & PAIR_ONE)) continue;
+                const cplx<R> v = rhoS[2 * f + e];
+                const size_t ge = base + cs(j + e) + i;
+                if (comp) {
+                    const float2 l = unpack_bf16x2(loS[2 * f + e]);
+                    a.state64[ge] = cplx<double>{(double)v.re + (double)l.x, (double)v.im + (double)l.y};
+                } else {
+                    a.state[ge] = v;
+                }
+            }
+        }
+        cl.sync();            // the other CTA has finished with this trajectory too
+    }
+}
+
 }  // namespace fpsg

@@ -47,6 +47,15 @@ struct QuadCfg {
     int nh = 2;             // k_resident_quad_hp: CTAs per spin (1: 2-CTA clusters)
 };
 
+// k_pair_packed; ept counts slots per thread, fn[0..1] is for 2 and 3 offsets
+template <typename R>
+const std::vector<QuadCfg<R>>& packed_cfgs();
+
+template <>
+const std::vector<QuadCfg<float>>& packed_cfgs<float>();
+template <>
+const std::vector<QuadCfg<double>>& packed_cfgs<double>();
+
 // index of a compact column width in QuadCfg::fn (-1: wider than supported)
 inline int quad_w_index(int W) { return W <= 5 ? 0 : W <= 9 ? 1 : W <= 13 ? 2 : W <= 17 ? 3 : -1; }
 
@@ -77,6 +86,8 @@ const std::vector<QuadCfg<double>>& quad_hp_cfgs<double>();
 #define FPSG_PAIR(R, NT, SPT, SPLIT)                                                  \
     {NT, SPT, SPLIT, {k_pair<R, NT, SPT, SPLIT, 2>, k_pair<R, NT, SPT, SPLIT, 3>},  \
      {k_pair<R, NT, SPT, SPLIT, 2, true>, k_pair<R, NT, SPT, SPLIT, 3, true>}}
+
+#define FPSG_PACKED(R, NT, SPT) {NT, SPT, {k_pair_packed<R, NT, SPT, 2>, k_pair_packed<R, NT, SPT, 3>}, {}, 1}
 
 #define FPSG_QUAD(R, NT, EPT)                                                                     \
     {NT, EPT, {k_resident_quad<R, NT, EPT, 5>, k_resident_quad<R, NT, EPT, 9>, k_resident_quad<R, NT, EPT, 13>, \

@@ -72,3 +72,48 @@ def test_pattern_needs_one_value():
     ref, out = compare(T, E.COUL_ONSITE, True, 3)
     assert np.array_equal(out[E.PREC_FP64][1], ref["final"])
 
+
+@pytest.mark.parametrize("dims,coulomb,ext,B,fp32", [
+    ((10, 7, 1), E.COUL_ONSITE, True, 3, False),     # 70: past the single-CTA and 2-CTA FP64 kernels
+    ((5, 5, 4), E.COUL_DISTANCE, False, 2, False),   # 100, three offsets
+    ((10, 10, 1), E.COUL_ONSITE, True, 35, False),   # more trajectories than clusters
+    ((11, 10, 1), E.COUL_ONSITE, True, 2, True),     # FP32 past k_pair
+    ((11, 11, 1), E.COUL_DISTANCE, False, 2, True),
+    ((12, 12, 1), E.COUL_ONSITE, False, 2, True),    # past k_pair_packed
+    ((101, 1, 1), E.COUL_ONSITE, False, 2, False),   # FP64 past it
+])
+def test_packed_matches_oracle(dims, coulomb, ext, B, fp32):
+    """k_pair_packed: FP64 to the bit, FP32 within the bound above; past it, the kernels of
+    two CTAs per spin."""
+    T = lattice(*dims, -1.0)
+    n = T.shape[0]
+    ref, out = compare(T, coulomb, ext, B, S=1, Tp=3) if not fp32 else compare_fp32(T, coulomb, ext, B)
+    if not fp32:
+        r, state = out[E.PREC_FP64]
+        assert np.array_equal(state, ref["final"])
+        for k in ("niiu", "n2iid", "nund", "energies"):
+            assert np.allclose(getattr(r, k), ref[k], rtol=1e-13, atol=1e-13), k
+    r, state = out[E.PREC_FP32]
+    assert np.max(np.abs(state - ref["final"])) < 12 * 0.2 * 8 * 2.0 * 2.0 ** -24 * 4
+    assert np.allclose(r.energies, ref["energies"], rtol=1e-6, atol=1e-6 * n)
+
+
+def compare_fp32(T, coulomb, ext, B):
+    """compare() without the FP64 run, which may be past the resident kernels."""
+    n = T.shape[0]
+    rng = np.random.default_rng(5)
+    D = np.abs(np.arange(n)[:, None] - np.arange(n)[None, :])
+    U = 2.0 / (1.0 + D) if coulomb == E.COUL_DISTANCE else np.diag(rng.uniform(1.0, 4.0, n))
+    V = U - np.diag(np.diag(U)) if coulomb == E.COUL_DISTANCE else None
+    X = np.diag(rng.uniform(-1, 1, n)) if ext else None
+    occ = (rng.random(n) < 0.5).astype(float)
+    rho = orc.sample(n, B, 11, occ, 1.0 - occ)
+    ref = orc.run(orc.System(T, U, V, X, coulomb, X is None), 0, 0.01, 1, 3, rho)
+    eng = E.Engine()
+    eng.set_system(T, U, V, X, coulomb)
+    eng.set_initial_samples(rho)
+    r = eng.run(E.METHOD_FTWA, E.PREC_FP32, 0.01, 1, 3)
+    assert r.path_used == E.PATH_RESIDENT
+    state = eng.get_state()
+    eng.close()
+    return ref, {E.PREC_FP32: (r, state)}
