@@ -20,6 +20,7 @@
 #include "fpsg_resident.h"
 #include "fpsg_util_kernels.cuh"
 #include "fpsg_adjoint.cuh"
+#include "fpsg_fock.cuh"
 #include "fpsg_gpsr.cuh"
 #include "fpsg_dense.h"
 
@@ -787,6 +788,53 @@ struct ResLauncher {
     }
 };
 
+// The cluster kernel of HF with the Fock term (fpsg_fock.cuh): the widest cluster the
+// device takes (16 CTAs, 8 per spin; else 8) whose slots cover the matrix, with X (and
+// Delta, where it fits too) in shared memory: n <= 84 in FP64 with both, n <= 119 with X
+// alone.  Larger systems run k_fock_stage.
+template <typename R>
+struct FockLauncher {
+    void (*fn)(FockRunArgs<R>) = nullptr;
+    int cps = 0, ncl = 0;
+    size_t smem = 0;
+    bool d_smem = false, tv_smem = false;
+
+    cudaLaunchConfig_t config(fpsg_ctx* ctx, int clusters, cudaLaunchAttribute* at) const
+    {
+        cudaLaunchConfig_t lc = {};
+        lc.gridDim = dim3(2 * cps * clusters); lc.blockDim = dim3(FOCK_NT); lc.dynamicSmemBytes = smem;
+        lc.stream = ctx->stream;
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 2 * cps; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        lc.attrs = at; lc.numAttrs = 1;
+        return lc;
+    }
+    bool setup(fpsg_ctx* ctx, int B)
+    {
+        d_smem = fock_layout<R>(ctx->n, true, false).total <= ctx->smem_optin;
+        tv_smem = fock_layout<R>(ctx->n, d_smem, true).total <= ctx->smem_optin;
+        tv_smem = tv_smem && d_smem;
+        smem = fock_layout<R>(ctx->n, d_smem, tv_smem).total;
+        if (smem > ctx->smem_optin) return false;
+        fn = tv_smem ? k_fock_run<R, true, true> : d_smem ? k_fock_run<R, true, false> : k_fock_run<R, false, false>;
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+            cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        for (int c : {8, 4}) {
+            if (ctx->n_pair > c * FOCK_NT) continue;
+            cps = c;
+            cudaLaunchAttribute at[1];
+            const cudaLaunchConfig_t lc = config(ctx, B, at);
+            if (cudaOccupancyMaxActiveClusters(&ncl, (void*)fn, &lc) != cudaSuccess) { cudaGetLastError(); ncl = 0; }
+            ncl = std::min(ncl, B);
+            if (ncl > 0) return true;
+        }
+        return false;
+    }
+};
+
 template <typename R>
 int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
 {
@@ -976,6 +1024,54 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
             CK(cudaStreamSynchronize(ctx->stream));
             fa.tMf = dt_; fa.Uf = du_; fa.Vf = dv_; fa.extf = de_; fa.D = dd_;
         }
+        FockLauncher<R> fl;
+        if (fock && ((size_t)q.Tp * B * 2 * (n + 4) * sizeof(double) >> 30) == 0 && fl.setup(ctx, B)) {
+            FockRunArgs<R> fr;
+            fr.sys = sys; fr.tMf = fa.tMf; fr.Uf = fa.Uf; fr.Vf = fa.Vf; fr.extf = fa.extf;
+            fr.uv_same = fr.ext_diag = 1;
+            for (int j = 0; j < n; ++j)
+                for (int i = 0; i < n; ++i) {
+                    const size_t x = (size_t)j * n + i;
+                    if (i != j && (R)ctx->U[x] != (R)ctx->V[x]) fr.uv_same = 0;
+                    if (i != j && !ctx->ext_null && (R)ctx->ext[x] != R(0)) fr.ext_diag = 0;
+                }
+            fr.state = st; fr.Dg = nullptr; fr.B = B; fr.cps = fl.cps; fr.h = (R)h; fr.hf = q.record;
+            fr.S = q.record ? q.S : 1; fr.Tp = q.record ? q.Tp : 1 << 30;
+            fr.record = q.record; fr.do_en = rec_e; fr.do_e1 = do_e1 && rec_e; fr.do_e2 = do_e2 && rec_e;
+            fr.diagbuf = nullptr; fr.ebuf = nullptr; fr.whole = whole; fr.order = ctx->pair_order;
+            fr.nslots = ctx->n_pair; fr.err = d_err;
+            double* fpart = nullptr;
+            const size_t eb = sizeof(double) * (size_t)q.Tp * B * 2 * 4;
+            if (!fl.d_smem && (rc = tmp((void**)&fr.Dg, sizeof(cplx<R>) * (size_t)2 * B * n * (n | 1)))) { cleanup(); return rc; }
+            if (q.record) {
+                if ((rc = tmp((void**)&fr.diagbuf, sizeof(double) * (size_t)q.Tp * B * 2 * n)) ||
+                    (rc = tmp((void**)&fr.ebuf, eb)) ||
+                    (rc = tmp((void**)&fpart, sizeof(double) * (size_t)q.Tp * nch * W))) {
+                    cleanup(); return rc;
+                }
+                CK(cudaMemsetAsync(fr.ebuf, 0, eb, ctx->stream));
+            }
+            cudaLaunchAttribute at[1];
+            const cudaLaunchConfig_t lc = fl.config(ctx, fl.ncl, at);
+            // time chunks, so that one launch stays in the tens of milliseconds
+            const long per_launch = std::max<long>(1, 4096 / ((B + fl.ncl - 1) / fl.ncl));
+            const int t_total = q.record ? q.Tp : q.n_steps;
+            const int tch = (int)std::max<long>(1, per_launch / fr.S);
+            long done = 0;
+            for (int t0 = 0; t0 < t_total; t0 += tch) {
+                fr.t_begin = t0; fr.t_end = std::min(t_total, t0 + tch);
+                fr.ptab = ptab ? ptab + done * 4 : nullptr;
+                CK(cudaLaunchKernelEx(&lc, fl.fn, fr));
+                out.launches++;
+                for (int t = t0; t < fr.t_end; ++t) done += (q.record && t == q.Tp - 1) ? 0 : fr.S;
+            }
+            if (q.record) {
+                k_reduce_part<<<dim3(nch, q.Tp), 256, 0, ctx->stream>>>(fr.diagbuf, fr.ebuf, B, n, chunk, fpart);
+                k_reduce_fin<<<dim3(std::max(1, (W + 255) / 256), q.Tp), 256, 0, ctx->stream>>>(fpart, nch, W, sums);
+                CK(cudaGetLastError());
+                out.launches += 2;
+            }
+        } else {
         const int fgrid = std::max(1, std::min(2 * B, 4 * ctx->sm_count));
         long gstep = 0;
         auto do_step = [&](bool record_now, double2* wslot) -> int {
@@ -1022,6 +1118,7 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
         } else {
             for (long s = 0; s < q.n_steps; ++s)
                 if ((rc = do_step(false, nullptr))) { cleanup(); return rc; }
+        }
         }
     }
     CK(cudaEventRecord(ctx->ev1, ctx->stream));

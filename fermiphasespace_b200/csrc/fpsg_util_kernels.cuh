@@ -7,12 +7,16 @@
 namespace fpsg {
 
 // ---- per-snapshot fixed-order reduction of the per-trajectory buffers
-// part[c][w] = sum over trajectories of chunk c (ascending) of the record values.
+// part[c][w] = sum over trajectories of chunk c (ascending) of the record values; block
+// row y takes the y-th snapshot of buffers that hold several.
 __global__ void k_reduce_part(const double* __restrict__ diagbuf, const double* __restrict__ ebuf,
                               int B, int n, int chunk, double* __restrict__ part)
 {
     const int W = rec_width(n);
     const int c = blockIdx.x;
+    diagbuf += (size_t)blockIdx.y * B * 2 * n;
+    ebuf += (size_t)blockIdx.y * B * 2 * 4;
+    part += (size_t)blockIdx.y * gridDim.x * W;
     const int b0 = c * chunk, b1 = min(B, b0 + chunk);
     for (int w = threadIdx.x; w < W; w += blockDim.x) {
         double acc = 0.0;
@@ -31,9 +35,11 @@ __global__ void k_reduce_part(const double* __restrict__ diagbuf, const double* 
     }
 }
 
-// out[w] = Kahan sum over c of part[c][w] (c ascending)
+// out[w] = Kahan sum over c of part[c][w] (c ascending), block row y: snapshot y
 __global__ void k_reduce_fin(const double* __restrict__ part, int nchunks, int W, double* __restrict__ out)
 {
+    part += (size_t)blockIdx.y * nchunks * W;
+    out += (size_t)blockIdx.y * W;
     for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < W; w += gridDim.x * blockDim.x) {
         double s = 0.0, comp = 0.0;
         for (int c = 0; c < nchunks; ++c) {

@@ -1,0 +1,51 @@
+"""The cluster kernel of HF with the Fock term against the oracle, at the sizes where its
+chunks, clusters and the place of Delta change."""
+import numpy as np
+import pytest
+
+from fermiphasespace_b200 import configs as cf
+from fermiphasespace_b200 import engine as E
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dims,B,S,Tp", [
+    ((1, 1), 1, 1, 3), ((2, 1), 3, 2, 3), ((3, 3), 12, 1, 4), ((8, 4), 1, 2, 3), ((11, 3), 2, 1, 3),
+    ((8, 8), 1, 1, 3),
+    ((9, 9), 1, 1, 2),       # Delta still in shared memory
+    ((10, 9), 1, 1, 2),      # Delta in global memory
+    ((17, 7), 1, 1, 2),      # the largest X
+    ((12, 10), 1, 1, 2),     # beyond: the per-stage kernel
+])
+def test_fock_matches_oracle(dims, B, S, Tp):
+    D = cf.distances(cf.grid_positions(*dims))
+    n = D.shape[0]
+    T = cf.hopping(D, [(1.0, -1.0)])
+    U = 2.0 / (1.0 + D)
+    V = U - np.diag(np.diag(U))
+    rng = np.random.default_rng(n)
+    ext = np.diag(rng.uniform(-1, 1, n))
+    rho = np.zeros((B, 2, n, n), dtype=complex)
+    for b in range(B):
+        for s in range(2):
+            _, R = np.linalg.eigh(T + np.diag(rng.uniform(-1, 1, n)))
+            rho[b, s] = R[:, : (n + 1 - s) // 2] @ R[:, : (n + 1 - s) // 2].T
+    rho = (rho + np.conj(np.swapaxes(rho, 2, 3))) / 2
+    ref = orc.run(orc.System(T, U, V, ext, orc.COUL_DISTANCE, False), 1, 0.01, S, Tp, rho)
+    eng = E.Engine()
+    eng.set_system(T, U, V, ext, E.COUL_DISTANCE)
+    eng.set_initial_samples(rho)
+    r = eng.run(E.METHOD_HF, E.PREC_FP64, 0.01, S, Tp)
+    assert r.path_used == E.PATH_STREAM
+    assert np.array_equal(eng.get_state(), ref["final"])
+    for k in ("niiu", "niid", "n2iiu", "n2iid", "nund"):
+        assert np.array_equal(getattr(r, k), ref[k]), k
+    # sums of n^2 terms of order 1 in another order
+    assert np.max(np.abs(r.energies - ref["energies"])) < 4 * n * n * 2.0 ** -52 * np.abs(ref["energies"]).max()
+    eng.set_initial_samples(rho)
+    r32 = eng.run(E.METHOD_HF, E.PREC_FP32, 0.01, S, Tp)
+    # FP32: S (Tp - 1) steps of 4 stages, |h Delta| <= 0.1, n-term sums of |X| <= 1, the state rounded every step
+    bound = S * (Tp - 1) * (4 * 0.1 * 4 * np.sqrt(n) + 4) * 2.0 ** -24 * 4
+    assert np.max(np.abs(r32.niiu - ref["niiu"])) < bound
+    eng.close()
