@@ -23,6 +23,7 @@
 #include "fpsg_fock.cuh"
 #include "fpsg_gpsr.cuh"
 #include "fpsg_dense.h"
+#include "fpsg_stream_pair.cuh"
 
 using namespace fpsg;
 
@@ -998,6 +999,21 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
         int per_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stage_fn, 256, smem));
         const int grid = std::max(1, std::min(2 * B, std::max(1, per_sm) * ctx->sm_count));
+        // With an offset pattern the pair stage, where a matrix has work for its 512 threads: it
+        // takes 0.3 ms per stage against 0.7 (n = 256, FP32, 512 trajectories), and in shared
+        // memory too k_stream_stage is the slower one (n = 143, FP64, 300 trajectories: 0.51
+        // against 0.25 ms).
+        const DevTables<R>& tb = tables<R>(ctx);
+        const bool sp = !fock && tb.pat_ns != 0 && (gx || ctx->n_pair >= 2 * SP_NT);
+        auto sp_fn = tb.pat_ns == 3 ? k_stream_pair<R, 3> : k_stream_pair<R, 2>;
+        const size_t sp_smem = stream_pair_smem(n, sizeof(R));
+        int sp_grid = 1;
+        if (sp) {
+            CK(cudaFuncSetAttribute(sp_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp_smem));
+            int occ = 0;
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sp_fn, SP_NT, sp_smem));
+            sp_grid = std::max(1, std::min(2 * B, std::max(1, occ) * ctx->sm_count));
+        }
         StreamArgs<R> sa;
         sa.sys = sys; sa.rho = st; sa.A = A; sa.Bc = Bc; sa.B = B; sa.h = (R)h;
         sa.do_e1 = do_e1 && rec_e; sa.do_e2 = do_e2 && rec_e;
@@ -1066,7 +1082,7 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
                 for (int t = t0; t < fr.t_end; ++t) done += (q.record && t == q.Tp - 1) ? 0 : fr.S;
             }
             if (q.record) {
-                k_reduce_part<<<dim3(nch, q.Tp), 256, 0, ctx->stream>>>(fr.diagbuf, fr.ebuf, B, n, chunk, fpart);
+                k_reduce_part<<<dim3(nch, q.Tp, (W + 255) / 256), 256, 0, ctx->stream>>>(fr.diagbuf, fr.ebuf, B, n, chunk, fpart);
                 k_reduce_fin<<<dim3(std::max(1, (W + 255) / 256), q.Tp), 256, 0, ctx->stream>>>(fpart, nch, W, sums);
                 CK(cudaGetLastError());
                 out.launches += 2;
@@ -1085,6 +1101,10 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
                 if (fock) {
                     fa.s = sa;
                     k_fock_stage<R><<<fgrid, 256, 0, ctx->stream>>>(fa);
+                } else if (sp) {
+                    StreamPairArgs<R> pa;
+                    pa.s = sa; pa.pat = tb.pat; pa.order = ctx->pair_order; pa.nslots = ctx->n_pair;
+                    sp_fn<<<sp_grid, SP_NT, sp_smem, ctx->stream>>>(pa);
                 } else {
                     stage_fn<<<grid, 256, smem, ctx->stream>>>(sa);
                 }
@@ -1095,7 +1115,7 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
             return FPSG_OK;
         };
         auto reduce_snapshot = [&](int t) -> int {
-            k_reduce_part<<<nch, 256, 0, ctx->stream>>>(diagbuf, ebuf, B, n, chunk, part);
+            k_reduce_part<<<dim3(nch, 1, (W + 255) / 256), 256, 0, ctx->stream>>>(diagbuf, ebuf, B, n, chunk, part);
             k_reduce_fin<<<std::max(1, (W + 255) / 256), 256, 0, ctx->stream>>>(part, nch, W, sums + (size_t)t * W);
             CK(cudaGetLastError());
             out.launches += 2;
@@ -1230,7 +1250,7 @@ int dense_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
             (rc = tmp((void**)&diagbuf, sizeof(double) * (size_t)B * 2 * n)) ||
             (rc = tmp((void**)&ebuf, sizeof(double) * (size_t)B * 2 * 4)) ||
             (rc = tmp((void**)&part, sizeof(double) * (size_t)nch * W)) ||
-            (rc = tmp((void**)&packed, sizeof(cplx<float>) * (size_t)M * ne))) {
+            ((q.obs & FPSG_OBS_WHOLE) && (rc = tmp((void**)&packed, sizeof(cplx<float>) * (size_t)M * ne)))) {
             cleanup();
             return rc;
         }
@@ -1269,12 +1289,41 @@ int dense_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
         tc += h;
         return FPSG_OK;
     };
+    // tM and the static potential in plane order, for the records
+    DenseRecordArgs dr = {};
+    if (q.record && !whole) {
+        std::vector<float> th((size_t)NP * NP, 0.f), eh((size_t)NP * NP, 0.f);
+        for (int j = 0; j < n; ++j)
+            for (int i = 0; i < n; ++i) {
+                th[plane_off(i, j)] = (float)ctx->tM[(size_t)j * n + i];
+                if (!ctx->ext_null) eh[plane_off(i, j)] = (float)ctx->ext[(size_t)j * n + i];
+            }
+        float *tt = nullptr, *et = nullptr;
+        if ((rc = tmp((void**)&tt, sizeof(float) * th.size())) ||
+            (!ctx->ext_null && (rc = tmp((void**)&et, sizeof(float) * eh.size())))) {
+            cleanup();
+            return rc;
+        }
+        CK(cudaMemcpyAsync(tt, th.data(), sizeof(float) * th.size(), cudaMemcpyHostToDevice, ctx->stream));
+        if (et) CK(cudaMemcpyAsync(et, eh.data(), sizeof(float) * eh.size(), cudaMemcpyHostToDevice, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        dr.n = n; dr.B = B; dr.X = R; dr.Tt = tt; dr.Et = et; dr.Ud = Ud; dr.Vd = Vd; dr.sys = sys;
+        dr.do_en = rec_e; dr.do_e1 = sa.do_e1; dr.do_e2 = sa.do_e2; dr.diagbuf = diagbuf; dr.ebuf = ebuf; dr.err = d_err;
+    }
     auto record = [&](int t) -> int {
+        if (!whole) {
+            CK(launch_record(dr, ctx->stream));
+            k_reduce_part<<<dim3(nch, 1, (W + 255) / 256), 256, 0, ctx->stream>>>(diagbuf, ebuf, B, n, chunk, part);
+            k_reduce_fin<<<std::max(1, (W + 255) / 256), 256, 0, ctx->stream>>>(part, nch, W, sums + (size_t)t * W);
+            CK(cudaGetLastError());
+            out.launches += 3;
+            return FPSG_OK;
+        }
         CK(pack_f32(R, n, M, packed, ctx->stream));
         sa.Xc = packed; sa.record = 1;
         sa.whole = whole ? whole + (size_t)t * 2 * ne : nullptr;
         k_stream_record<float><<<rgrid, 256, 0, ctx->stream>>>(sa);
-        k_reduce_part<<<nch, 256, 0, ctx->stream>>>(diagbuf, ebuf, B, n, chunk, part);
+        k_reduce_part<<<dim3(nch, 1, (W + 255) / 256), 256, 0, ctx->stream>>>(diagbuf, ebuf, B, n, chunk, part);
         k_reduce_fin<<<std::max(1, (W + 255) / 256), 256, 0, ctx->stream>>>(part, nch, W, sums + (size_t)t * W);
         CK(cudaGetLastError());
         out.launches += 4;
@@ -1459,7 +1508,7 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
         return cudaGetLastError() == cudaSuccess ? FPSG_OK : fail(ctx, FPSG_ERR_CUDA, "adjoint forward stage launch failed");
     };
     auto reduce_snapshot = [&](int t) {
-        k_reduce_part<<<nch, 256, 0, ctx->stream>>>(diagbuf, ebuf, B, n, chunk, part);
+        k_reduce_part<<<dim3(nch, 1, (W + 255) / 256), 256, 0, ctx->stream>>>(diagbuf, ebuf, B, n, chunk, part);
         k_reduce_fin<<<std::max(1, (W + 255) / 256), 256, 0, ctx->stream>>>(part, nch, W, sums + (size_t)t * W);
     };
 
@@ -2134,7 +2183,7 @@ int batch_impl(fpsg_ctx* ctx, const fpsg_system_desc* sd, int ns, int method, do
             }
         for (int l = 0; l < nss; ++l) {
             SysBuf& b = sb[l];
-            k_reduce_part<<<b.nch, 256, 0, ctx->stream>>>(b.diagbuf, b.ebuf, b.B, b.n, chunk, b.part);
+            k_reduce_part<<<dim3(b.nch, 1, (b.W + 255) / 256), 256, 0, ctx->stream>>>(b.diagbuf, b.ebuf, b.B, b.n, chunk, b.part);
             k_reduce_fin_at<<<std::max(1, (b.W + 255) / 256), 256, 0, ctx->stream>>>(b.part, b.nch, b.W, b.sums, t_ctr);
             nodes += 2;
         }
@@ -2162,7 +2211,7 @@ int batch_impl(fpsg_ctx* ctx, const fpsg_system_desc* sd, int ns, int method, do
             for (int l = 0; l < nss; ++l) {
                 SysBuf& b = sb[l];
                 k_stream_record<R><<<std::max(1, std::min(2 * b.B, 4 * ctx->sm_count)), 256, 0, ctx->stream>>>(ha[l]);
-                k_reduce_part<<<b.nch, 256, 0, ctx->stream>>>(b.diagbuf, b.ebuf, b.B, b.n, chunk, b.part);
+                k_reduce_part<<<dim3(b.nch, 1, (b.W + 255) / 256), 256, 0, ctx->stream>>>(b.diagbuf, b.ebuf, b.B, b.n, chunk, b.part);
                 k_reduce_fin_at<<<std::max(1, (b.W + 255) / 256), 256, 0, ctx->stream>>>(b.part, b.nch, b.W, b.sums, t_ctr);
                 launches += 3;
             }

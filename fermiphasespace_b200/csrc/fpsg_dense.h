@@ -51,10 +51,26 @@ struct DenseArgs {
     uint32_t probe_polls = 0;
 };
 
+// Arguments of one snapshot record over all trajectories (diagonals and energy rows).
+struct DenseRecordArgs {
+    int n, B;
+    const float* X;              // state planes
+    const float* Tt;             // tM, and the static potential (null: none), FP32 in plane order
+    const float* Et;
+    const float* Ud;             // dense U, V ([NP][NP]) for long-range Coulomb, else null (index lists of sys)
+    const float* Vd;
+    DevSys<float> sys;
+    int do_en, do_e1, do_e2;
+    double* diagbuf;             // [B][2][n]
+    double* ebuf;                // [B][2][4]
+    unsigned* err;
+};
+
 size_t stage_smem_bytes();
 int stage_threads();
 cudaError_t configure();                                        // opt-in shared memory
 cudaError_t launch_stage(const DenseArgs& a, int grid, bool tf32, cudaStream_t st);
+cudaError_t launch_record(const DenseRecordArgs& a, cudaStream_t st);
 // T ([NP][NP] FP32 device, diagonal dropped) -> canonical two-term tiles of the mode
 cudaError_t prep_T(const float* T_full, void* Tc, bool tf32, cudaStream_t st);
 // packed FP64 state [M][ne] complex -> full FP32 planes

@@ -8,7 +8,7 @@ namespace fpsg {
 
 // ---- per-snapshot fixed-order reduction of the per-trajectory buffers
 // part[c][w] = sum over trajectories of chunk c (ascending) of the record values; block
-// row y takes the y-th snapshot of buffers that hold several.
+// row y takes the y-th snapshot of buffers that hold several, z a share of the values.
 __global__ void k_reduce_part(const double* __restrict__ diagbuf, const double* __restrict__ ebuf,
                               int B, int n, int chunk, double* __restrict__ part)
 {
@@ -18,7 +18,7 @@ __global__ void k_reduce_part(const double* __restrict__ diagbuf, const double* 
     ebuf += (size_t)blockIdx.y * B * 2 * 4;
     part += (size_t)blockIdx.y * gridDim.x * W;
     const int b0 = c * chunk, b1 = min(B, b0 + chunk);
-    for (int w = threadIdx.x; w < W; w += blockDim.x) {
+    for (int w = blockIdx.z * blockDim.x + threadIdx.x; w < W; w += gridDim.z * blockDim.x) {
         double acc = 0.0;
         if (w < 5 * n) {
             const int o = w / n, j = w - o * n;
