@@ -1610,22 +1610,37 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
         egrid = std::max(1, std::min(2 * B, std::max(1, per_sm) * ctx->sm_count));
     }
     const R hR = (R)h;
-    // the segment-resident reverse kernel: on-site (or no) Coulomb term, fixed-width
-    // columns with P <= 4, the packed matrix within 512 x 5 slots
-    constexpr int SEG_NT = 512, SEG_EPT = 5;
-    const bool use_seg = plan.idx >= 0 && tables<R>(ctx).dd_fusable && (ellP == 2 || ellP == 4) &&
-                         ne <= SEG_NT * SEG_EPT &&
-                         (ellP == 2 ? vjp_seg_smem<R, 2>(n, ne, nb) : vjp_seg_smem<R, 4>(n, ne, nb)) <= ctx->smem_optin;
-    auto seg_fn = ellP == 2 ? k_vjp_segment<R, SEG_NT, SEG_EPT, 2> : k_vjp_segment<R, SEG_NT, SEG_EPT, 4>;
+    // the segment-resident reverse kernel: on-site (or no) Coulomb term, an offset pattern or
+    // fixed-width columns with P <= 4, the packed matrix within the slots of a configuration;
+    // the smallest one that holds it (5x5 grid, FP64, 300 trajectories, ten steps: 545 us with
+    // 512 threads per CTA, 128 with 128)
+    const DevTables<R>& tv = tables<R>(ctx);
+    const int seg_v = tv.pat_ns && n < 256 ? tv.pat_ns : ellP == 2 ? 0 : 1;
+    const VjpCfg<R>* seg_cfg = nullptr;
+    for (const VjpCfg<R>& c : vjp_cfgs<R>())
+        if (!seg_cfg && c.nt * c.ept >= ne && n <= c.nt) seg_cfg = &c;
+    auto seg_bytes = [&](bool xs) -> size_t {
+        const int mo = tv.pat.off[0];
+        switch (seg_v) {
+        case 0: return xs ? vjp_seg_smem<R, 2, true>(n, ne, nb, mo) : vjp_seg_smem<R, 2>(n, ne, nb, mo);
+        case 1: return xs ? vjp_seg_smem<R, 4, true>(n, ne, nb, mo) : vjp_seg_smem<R, 4>(n, ne, nb, mo);
+        case 2: return xs ? vjp_seg_smem<R, -2, true>(n, ne, nb, mo) : vjp_seg_smem<R, -2>(n, ne, nb, mo);
+        default: return xs ? vjp_seg_smem<R, -3, true>(n, ne, nb, mo) : vjp_seg_smem<R, -3>(n, ne, nb, mo);
+        }
+    };
+    const bool use_seg = plan.idx >= 0 && tv.dd_fusable && seg_cfg && (seg_v >= 2 || ellP == 2 || ellP == 4) &&
+                         seg_bytes(false) <= ctx->smem_optin;
+    const int SEG_NT = seg_cfg ? seg_cfg->nt : 0;
+    ResKernelVjp<R> seg_fn = seg_cfg ? seg_cfg->fn[0][seg_v] : nullptr;
     VjpSegArgs<R> vs;
     int seg_grid = 0;
     size_t seg_smem = 0;
     if (use_seg) {
-        // two variants: stage adjoints in registers (one cluster per SM pair) or in
-        // shared memory (64 registers, two clusters per SM pair when they fit)
-        auto seg_fn_xs = ellP == 2 ? k_vjp_segment<R, SEG_NT, SEG_EPT, 2, true> : k_vjp_segment<R, SEG_NT, SEG_EPT, 4, true>;
-        const size_t smem_xs = ellP == 2 ? vjp_seg_smem<R, 2, true>(n, ne, nb) : vjp_seg_smem<R, 4, true>(n, ne, nb);
-        seg_smem = ellP == 2 ? vjp_seg_smem<R, 2>(n, ne, nb) : vjp_seg_smem<R, 4>(n, ne, nb);
+        // two variants: stage adjoints in registers (128 per thread) or in shared memory
+        // (64 registers, twice the clusters where they fit)
+        const ResKernelVjp<R> seg_fn_xs = seg_cfg->fn[1][seg_v];
+        const size_t smem_xs = seg_bytes(true);
+        seg_smem = seg_bytes(false);
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
@@ -1641,7 +1656,7 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
         };
         int ncl = 0, ncl_xs = 0;
         if ((rc = clusters(seg_fn, seg_smem, ncl)) || (rc = clusters(seg_fn_xs, smem_xs, ncl_xs))) { cleanup(); return rc; }
-        if (ncl_xs > ncl) { seg_fn = seg_fn_xs; seg_smem = smem_xs; ncl = ncl_xs; }
+        if (std::min(ncl_xs, B) > std::min(ncl, B)) { seg_fn = seg_fn_xs; seg_smem = smem_xs; ncl = ncl_xs; }
         seg_grid = 2 * std::max(1, std::min(B, ncl));
         double* envtab = nullptr;
         int* bintab = nullptr;
@@ -1664,7 +1679,7 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
         vs.ptab = ptab; vs.envtab = envtab; vs.bintab = bintab; vs.n_bins = nb;
         vs.h = hR; vs.S = S; vs.Tp = Tp; vs.dt = dt; vs.lscale = lscale;
         vs.ell_k = tables<R>(ctx).ell_k; vs.ell_v = tables<R>(ctx).ell_v; vs.order = ctx->res_order;
-        vs.udiag = tables<R>(ctx).udiag; vs.err = d_err;
+        vs.udiag = tables<R>(ctx).udiag; vs.pat = tv.pat; vs.err = d_err;
     }
 
     for (int b0 = 0; b0 < Ball; b0 += B) {
@@ -1792,7 +1807,7 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
         k_slot_reduce<<<std::max(1, std::min<int>((int)((TW + 255) / 256), ctx->sm_count * 4)), 256, 0, ctx->stream>>>(slots, rl.grid, TW, sums);
         CK(cudaGetLastError());
     }
-    k_pacc_reduce<<<1, 64, 0, ctx->stream>>>(pacc, Ball * 2, PW, pout);
+    k_pacc_reduce<<<PW, PACC_NT, 0, ctx->stream>>>(pacc, Ball * 2, PW, pout);
     CK(cudaEventRecord(ctx->ev1, ctx->stream));
     std::vector<double> hs((size_t)Tp * W), hp(PW);
     unsigned flag = 0;

@@ -16,6 +16,7 @@
 // two entries of the full matrix in inner products (weight 2).
 #pragma once
 #include "fpsg_kernels.cuh"
+#include "fpsg_pair.cuh"
 
 namespace fpsg {
 
@@ -307,21 +308,6 @@ __global__ void k_loss_grad(int n, int ne, int B, const cplx<R>* __restrict__ y,
     }
 }
 
-// parameter totals: out[c] = sum over trajectories and spins of pacc[.][c] (fixed order)
-__global__ void k_pacc_reduce(const double* __restrict__ pacc, int M, int W, double* __restrict__ out)
-{
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < W; c += gridDim.x * blockDim.x) {
-        double s = 0.0, comp = 0.0;
-        for (int m = 0; m < M; ++m) {
-            const double y = pacc[(size_t)m * W + c] - comp;
-            const double t = s + y;
-            comp = (t - s) - y;
-            s = t;
-        }
-        out[c] = s;
-    }
-}
-
 }  // namespace fpsg
 
 namespace fpsg {
@@ -365,6 +351,7 @@ struct VjpSegArgs {
     const R* ell_v;
     const uint32_t* order;     // element (i | j << 16) of each slot
     const R* udiag;            // U_jj
+    Pattern<R> pat;            // offset pattern (P < 0)
     unsigned* err;
 };
 
@@ -373,11 +360,19 @@ struct __align__(8) VEnt { int k; R v; };
 template <>
 struct __align__(16) VEnt<double> { int k; int pad; double v; };
 
-template <typename R, int P, bool XS = false>
-__host__ __device__ __forceinline__ size_t vjp_seg_smem(int n, int ne, int n_bins)
+// bytes in front of K that masked neighbours (P < 0: a pattern with -P offsets) may read
+template <typename R, int P>
+__host__ __device__ __forceinline__ size_t vjp_seg_guard(int n, int max_off)
 {
-    const int RPc = n | 1, NE = 2 * P + 1;
-    size_t o = sizeof(cplx<R>) * (size_t)n * RPc;          // K
+    return P < 0 ? align16(sizeof(cplx<R>) * (size_t)(n | 1) * max_off) : 0;
+}
+template <typename R, int P, bool XS = false>
+__host__ __device__ __forceinline__ size_t vjp_seg_smem(int n, int ne, int n_bins, int max_off)
+{
+    const int RPc = n | 1, NE = P < 0 ? 0 : 2 * P + 1;
+    size_t o = vjp_seg_guard<R, P>(n, max_off);
+    const size_t k_end = o + sizeof(cplx<R>) * (size_t)n * RPc;
+    o = k_end;                                              // K
     o = align16(o + sizeof(R) * (size_t)n * RPc);           // EP (full, signed)
     o = align16(o + sizeof(R) * (size_t)n * 3);             // Dd, xod, xo0
     o = align16(o + sizeof(R) * (size_t)n * 2);             // dbo[2]
@@ -388,16 +383,24 @@ __host__ __device__ __forceinline__ size_t vjp_seg_smem(int n, int ne, int n_bin
     o = align16(o + sizeof(double) * (size_t)(2 + n_bins)); // parameter partials of the trajectory
     o = align16(o + sizeof(double) * (size_t)(512 + 64 * 3)); // running partials per thread / column group
     if (XS) o += sizeof(cplx<R>) * 3 * (size_t)ne;          // stage adjoints 4, 3, 2 by slot
-    return o;
+    return o > k_end + vjp_seg_guard<R, P>(n, max_off) ? o : k_end + vjp_seg_guard<R, P>(n, max_off);
 }
 
 // XS = true keeps the stage adjoints 4, 3, 2 in shared memory (one slot per element,
-// thread-private) instead of registers, so that two clusters fit on an SM pair.
+// thread-private) instead of registers, so that two clusters fit on an SM pair.  P > 0:
+// fixed-width columns of P entries on each side of the diagonal; P < 0: an offset pattern
+// with -P offsets, whose terms are read at fixed distances in K under mask bits (see
+// fpsg_pair.cuh): no column entries (12 wavefronts per 32 elements at P = 2).  Smaller
+// systems take fewer threads per CTA, so that more trajectories are in flight.
+// Segments of 16 steps: VJP_MEASURED
 template <typename R, int NT, int EPT, int P, bool XS = false>
-__global__ void __launch_bounds__(NT, XS ? 2 : 1) k_vjp_segment(VjpSegArgs<R> a)
+__global__ void __launch_bounds__(NT, (XS ? 1024 : 512) / NT) k_vjp_segment(VjpSegArgs<R> a)
 {
-    extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int NE = 2 * P + 1, NW = NT / 32;
+    extern __shared__ __align__(16) unsigned char smem_all[];
+    constexpr bool PAT = P < 0;
+    constexpr int NS = PAT ? -P : 2;
+    constexpr int NE = PAT ? 0 : 2 * P + 1, NW = NT / 32;
+    unsigned char* smem = smem_all + vjp_seg_guard<R, P>(a.sys.n, PAT ? a.pat.off[0] : 0);
     const int n = a.sys.n, ne = a.sys.ne, RPc = n | 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     size_t o = sizeof(cplx<R>) * (size_t)n * RPc;
@@ -442,7 +445,7 @@ __global__ void __launch_bounds__(NT, XS ? 2 : 1) k_vjp_segment(VjpSegArgs<R> a)
     const int cid = blockIdx.x >> 1, ncl = gridDim.x >> 1;
     R* peer_dbo = cl.map_shared_rank(dbo, s ^ 1);
 
-    for (int q = tid; q < n * NE; q += NT) {
+    if constexpr (!PAT) for (int q = tid; q < n * NE; q += NT) {
         const int col = q / NE, sl = q - col * NE;
         const int k = a.ell_k[q];
         VEnt<R> e;
@@ -463,9 +466,13 @@ __global__ void __launch_bounds__(NT, XS ? 2 : 1) k_vjp_segment(VjpSegArgs<R> a)
     for (int q = 0; q < EPT; ++q) {
         const int f = tid + q * NT;
         ij[q] = f < ne ? a.order[f] : ~0u;
+        if (PAT && f < ne) {                         // i | j << 8 | masks of j, of i
+            const uint32_t i = ij[q] & 0xffffu, j = ij[q] >> 16;
+            ij[q] = i | (j << 8) | (a.pat.mask[j] << 16) | (a.pat.mask[i] << (16 + 2 * NS));
+        }
     }
-    auto I_ = [&](int q) { return (int)(ij[q] & 0xffffu); };
-    auto J_ = [&](int q) { return (int)(ij[q] >> 16); };
+    auto I_ = [&](int q) { return PAT ? (int)(ij[q] & 0xffu) : (int)(ij[q] & 0xffffu); };
+    auto J_ = [&](int q) { return PAT ? (int)((ij[q] >> 8) & 0xffu) : (int)(ij[q] >> 16); };
     auto P_ = [&](int q) { return cs(J_(q)) + I_(q); };
     const R hR = a.h;
     const double shift = (double)a.sys.shift;
@@ -569,6 +576,41 @@ __global__ void __launch_bounds__(NT, XS ? 2 : 1) k_vjp_segment(VjpSegArgs<R> a)
                     // per-stage kernels), FP32 adds Kb_ij (Delta_jj - Delta_ii) once afterwards
                     constexpr bool kDiagApart = std::is_same<R, float>::value;
                     R are = R(0), aim = R(0), bre = R(0), bim = R(0);
+                    if constexpr (PAT && kDiagApart) {
+                        const uint64_t* k0 = reinterpret_cast<const uint64_t*>(K + (size_t)j * RPc + i);
+                        uint64_t ga = 0, gb = 0;
+                        auto terms = [&](auto sc) {
+                            constexpr int u = decltype(sc)::value;
+                            const int o = u == NS - 1 && NS > 1 ? 1 : a.pat.off[u];
+                            f2_add_if<(1u << (16 + 2 * u))>(ga, k0[-o * RPc], ij[q]);
+                            f2_add_if<(1u << (16 + 2 * NS + 2 * u))>(gb, k0[-o], ij[q]);
+                            f2_add_if<(1u << (17 + 2 * u))>(ga, k0[o * RPc], ij[q]);
+                            f2_add_if<(1u << (17 + 2 * NS + 2 * u))>(gb, k0[o], ij[q]);
+                        };
+                        terms(std::integral_constant<int, 0>());
+                        terms(std::integral_constant<int, 1>());
+                        if constexpr (NS == 3) terms(std::integral_constant<int, 2>());
+                        const cplx<float> t = f2_unpack(f2_sub(ga, gb));
+                        are = t.re * a.pat.w;
+                        aim = t.im * a.pat.w;
+                    } else if constexpr (PAT) {
+                        const cplx<R>* k0 = K + (size_t)j * RPc + i;
+                        const uint32_t mj = ij[q] >> 16, mi = ij[q] >> (16 + 2 * NS);
+                        auto side = [&](int u) {
+#pragma unroll
+                            for (int t = 0; t < NS; ++t) {
+                                const int c = u ? NS - 1 - t : t, o = u ? a.pat.off[c] : -a.pat.off[c];
+                                const cplx<R> xa = k0[o * RPc], xc = k0[o];
+                                if ((mj >> (2 * c + u)) & 1u) { are = fmaR<R>(xa.re, a.pat.w, are); aim = fmaR<R>(xa.im, a.pat.w, aim); }
+                                if ((mi >> (2 * c + u)) & 1u) { bre = fmaR<R>(xc.re, a.pat.w, bre); bim = fmaR<R>(xc.im, a.pat.w, bim); }
+                            }
+                        };
+                        side(0);
+                        const R dj = Dd[j], di = Dd[i];
+                        are = fmaR<R>(kb.re, dj, are); aim = fmaR<R>(kb.im, dj, aim);
+                        bre = fmaR<R>(kb.re, di, bre); bim = fmaR<R>(kb.im, di, bim);
+                        side(1);
+                    } else {
 #pragma unroll
                     for (int sl = 0; sl < NE; ++sl) {          // sum_k Kb_ik Delta_kj over column j
                         if (kDiagApart && sl == P) continue;
@@ -586,6 +628,7 @@ __global__ void __launch_bounds__(NT, XS ? 2 : 1) k_vjp_segment(VjpSegArgs<R> a)
                         const cplx<R> x = K[(size_t)j * RPc + e.k];
                         bre = fmaR<R>(x.re, d, bre);
                         bim = fmaR<R>(x.im, d, bim);
+                    }
                     }
                     if constexpr (kDiagApart) {
                         const R dd = Dd[j] - Dd[i];

@@ -4,6 +4,7 @@
 #pragma once
 #include <vector>
 
+#include "fpsg_adjoint.cuh"
 #include "fpsg_kernels.cuh"
 #include "fpsg_pair.cuh"
 #include "fpsg_quad.cuh"
@@ -76,7 +77,30 @@ const std::vector<QuadCfg<float>>& quad_hp_cfgs<float>();
 template <>
 const std::vector<QuadCfg<double>>& quad_hp_cfgs<double>();
 
+// k_vjp_segment: threads per CTA and elements per thread; fn[x][v]: stage adjoints in
+// registers (x = 0) or shared memory (1), columns with P = 2, 4 (v = 0, 1) or an offset
+// pattern with 2, 3 offsets (2, 3)
+template <typename R>
+struct VjpCfg {
+    int nt, ept;
+    void (*fn[2][4])(VjpSegArgs<R>);
+};
+
+template <typename R>
+const std::vector<VjpCfg<R>>& vjp_cfgs();
+
+template <>
+const std::vector<VjpCfg<float>>& vjp_cfgs<float>();
+template <>
+const std::vector<VjpCfg<double>>& vjp_cfgs<double>();
+
 }  // namespace fpsg
+
+#define FPSG_VJP(R, NT, EPT)                                                                                   \
+    {NT, EPT, {{k_vjp_segment<R, NT, EPT, 2>, k_vjp_segment<R, NT, EPT, 4>, k_vjp_segment<R, NT, EPT, -2>,    \
+                k_vjp_segment<R, NT, EPT, -3>},                                                              \
+               {k_vjp_segment<R, NT, EPT, 2, true>, k_vjp_segment<R, NT, EPT, 4, true>,                      \
+                k_vjp_segment<R, NT, EPT, -2, true>, k_vjp_segment<R, NT, EPT, -3, true>}}}
 
 #define FPSG_RES(R, NT, EPT, SPLIT)                                                                           \
     {NT, EPT, SPLIT,                                                                                      \

@@ -269,3 +269,34 @@ def test_adjoint_full_shape_finite_differences(engine, engine_lib, oracle_lib):
     for k in ("dU", "dt"):
         assert abs(g32[k] - g[k]) < 2e-4 * abs(g[k]), (k, g32[k], g[k])
     assert np.abs(g32["dpulse"] - g["dpulse"]).max() < 5e-4 * np.abs(g["dpulse"]).max()
+
+
+@pytest.mark.parametrize("dims", [(1, 2), (3, 3), (26, 1), (27, 1), (28, 1), (4, 11), (5, 9), (8, 8), (4, 4, 4)])
+def test_segment_kernel_configurations(engine_lib, dims):
+    """Every configuration of the segment-resident reverse kernel (threads per CTA, pattern and
+    column variants) against the per-stage kernels, which a distance matrix with the same
+    on-site U and V = 0 takes: the same formulas, so FP64 agrees to rounding."""
+    E = engine_lib
+    pos = configs.grid_positions(*dims)
+    T = configs.hopping(configs.distances(pos), [(1.0, -1.0)])
+    n = T.shape[0]
+    rng = np.random.default_rng(n)
+    occ = (rng.random(n) < 0.5).astype(float)
+    U = np.diag(rng.uniform(2.0, 4.0, n))
+    X = np.diag(rng.uniform(-1, 1, n))
+    pulse = dict(amp=rng.normal(0, 0.5, 4), bin_width=0.05, t0=0.1, td=0.05, proj=pos[:, 0] - pos[:, 0].mean())
+    for tm in (T, T * np.where(np.abs(np.subtract.outer(np.arange(n), np.arange(n))) == 1, 1.0, 0.9)):
+        for prec, tol in ((E.PREC_FP64, 1e-11), (E.PREC_FP32, 2e-5)):
+            got = []
+            for coul, V in ((E.COUL_ONSITE, None), (E.COUL_DISTANCE, np.zeros((n, n)))):
+                eng = E.Engine()
+                eng.set_system(tm, U, V, X, coul)
+                eng.set_pulse(**pulse)
+                eng.sample(7, 5, occ, 1.0 - occ)
+                got.append(eng.grad(prec, 0.01, 2, 11, 4))
+                eng.close()
+            a, b = got
+            scale = max(abs(b["dU"]), abs(b["dt"]), np.abs(b["dpulse"]).max(), 1e-3)
+            assert abs(a["loss"] - b["loss"]) < tol
+            for k in ("dU", "dt", "dpulse"):
+                assert np.max(np.abs(a[k] - b[k])) < tol * scale, (k, prec)
