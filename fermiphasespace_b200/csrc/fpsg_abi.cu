@@ -77,6 +77,7 @@ struct fpsg_ctx {
     uint64_t mem_cap = 0, mem_used = 0;
     std::vector<DevAlloc> allocs;
     std::vector<DevAlloc> pool;            // per-call scratch kept for the next call (counted in mem_used)
+    bool pooled_state = false;             // the state comes from the pool (systems of a batch)
     int64_t grad_keep = -1;                // fpsg_set_grad_memory: -1 automatic
     fpsg_grad_info grad_info = {0, 0, 0, 0};   // the last fpsg_grad call's plan
 
@@ -652,7 +653,7 @@ ResPlan plan_packed(fpsg_ctx* ctx, bool comp)
     for (int c = 0; c < (int)cf.size(); ++c) {
         const int cap = cf[c].nt * cf[c].ept;
         if (cap < ctx->n_pair) continue;
-        const size_t sm = packed_layout<R>(ctx->n, cap, comp, t.pat.off[0], t.ud != nullptr).total;
+        const size_t sm = packed_layout<R>(ctx->n, ctx->n_pair, comp, t.pat.off[0], t.ud != nullptr).total;
         if (sm > ctx->smem_optin) continue;
         best.idx = c; best.G = 1; best.smem = sm; best.quad = best.pair = true; best.comp = comp; best.nh = 1;
         break;
@@ -1920,13 +1921,29 @@ void fill_outputs(int n, int ne, int B, int method, double dt, int S, int Tp, ui
 }
 
 // ------------------------------------------------------------------ batch
-// Releases the device memory of a context made for one system of a batch (its
-// stream and events belong to the parent).
-void release_sub(fpsg_ctx* c)
+// The context made for one system of a batch (its stream and events belong to the parent)
+// takes its device memory from the parent's pool and leaves it there afterwards, so that the
+// next batch of similar sizes allocates nothing: some 500 MB of states and ten table blocks
+// per call cost several ms of cudaMalloc and cudaFree otherwise.
+void lend_pool(fpsg_ctx* from, fpsg_ctx* to)
 {
-    for (auto& a : c->allocs) cudaFree(a.p);
-    c->allocs.clear();
-    c->pool.clear();
+    for (const DevAlloc& blk : from->pool) {
+        for (size_t i = 0; i < from->allocs.size(); ++i)
+            if (from->allocs[i].p == blk.p) {
+                from->allocs.erase(from->allocs.begin() + i);
+                break;
+            }
+        from->mem_used -= blk.bytes;
+        to->allocs.push_back(blk);
+        to->pool.push_back(blk);
+        to->mem_used += blk.bytes;
+    }
+    from->pool.clear();
+}
+void release_sub(fpsg_ctx* c, fpsg_ctx* parent)
+{
+    c->pool = c->allocs;          // everything it holds
+    lend_pool(c, parent);
 }
 
 template <typename R>
@@ -1949,8 +1966,9 @@ int batch_impl(fpsg_ctx* ctx, const fpsg_system_desc* sd, int ns, int method, do
         if (graph) cudaGraphDestroy(graph);
         if (rgexec) cudaGraphExecDestroy(rgexec);
         if (rgraph) cudaGraphDestroy(rgraph);
+        cudaStreamSynchronize(ctx->stream);     // pooled blocks may be written by the host next
         for (void* p : temps) trelease(ctx, p);
-        for (auto& c : subs) release_sub(c.get());
+        for (auto& c : subs) release_sub(c.get(), ctx);
     };
     // systems and their samples, each in a context of its own
     for (int k = 0; k < ns; ++k) {
@@ -1958,10 +1976,15 @@ int batch_impl(fpsg_ctx* ctx, const fpsg_system_desc* sd, int ns, int method, do
         fpsg_ctx* c = subs.back().get();
         c->device = ctx->device; c->sm_count = ctx->sm_count; c->smem_optin = ctx->smem_optin;
         c->stream = ctx->stream; c->ev0 = ctx->ev0; c->ev1 = ctx->ev1; c->flags = ctx->flags;
+        lend_pool(ctx, c);
+        c->pooled_state = true;
+        // what the parent holds beside its pool counts against the cap
         c->mem_cap = ctx->mem_cap ? (ctx->mem_cap > ctx->mem_used ? ctx->mem_cap - ctx->mem_used : 1) : 0;
         int rc = fpsg_set_system(c, sd[k].n, sd[k].tM, sd[k].U, sd[k].V, sd[k].extpot, sd[k].coulomb_kind,
                                  sd[k].extpot_is_null);
         if (!rc) rc = fpsg_sample(c, sd[k].n_traj, sd[k].seed, sd[k].occ_up, sd[k].occ_dn, nullptr, nullptr);
+        if (ctx->mem_cap) trim_pool(c);
+        lend_pool(c, ctx);
         if (rc) {
             const std::string why = c->err;
             cleanup();
@@ -2427,7 +2450,8 @@ static int alloc_state(fpsg_ctx* ctx, int B)
 {
     if (ctx->rho64 && ctx->B == B) return FPSG_OK;
     dfree(ctx, ctx->rho64); ctx->rho64 = nullptr; ctx->B = 0;
-    int rc = dalloc(ctx, (void**)&ctx->rho64, sizeof(cplx<double>) * (size_t)B * 2 * ctx->ne);
+    const size_t bytes = sizeof(cplx<double>) * (size_t)B * 2 * ctx->ne;
+    int rc = ctx->pooled_state ? talloc(ctx, (void**)&ctx->rho64, bytes) : dalloc(ctx, (void**)&ctx->rho64, bytes);
     if (rc) return rc;
     ctx->B = B;
     return FPSG_OK;

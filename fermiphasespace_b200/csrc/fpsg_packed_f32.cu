@@ -7,7 +7,7 @@ template <>
 const std::vector<QuadCfg<float>>& packed_cfgs<float>()
 {
     static const std::vector<QuadCfg<float>> v = {
-        FPSG_PACKED(float, 512, 6), FPSG_PACKED(float, 512, 8),
+        FPSG_PACKED(float, 512, 6, false), FPSG_PACKED(float, 512, 8, false), FPSG_PACKED(float, 512, 11, true),
     };
     return v;
 }

@@ -7,7 +7,7 @@ template <>
 const std::vector<QuadCfg<double>>& packed_cfgs<double>()
 {
     static const std::vector<QuadCfg<double>> v = {
-        FPSG_PACKED(double, 512, 3), FPSG_PACKED(double, 512, 4), FPSG_PACKED(double, 512, 5),
+        FPSG_PACKED(double, 512, 3, false), FPSG_PACKED(double, 512, 4, false), FPSG_PACKED(double, 512, 5, false),
     };
     return v;
 }

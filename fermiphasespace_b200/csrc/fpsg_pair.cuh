@@ -620,25 +620,28 @@ struct PackedAddr {
 };
 
 template <typename R>
-__host__ __device__ __forceinline__ ResLayout<R> packed_layout(int n, int slots, bool comp, int D, bool dense_coul)
+__host__ __device__ __forceinline__ ResLayout<R> packed_layout(int n, int nslots, bool comp, int D, bool dense_coul)
 {
     ResLayout<R> L;
-    // masked neighbours: C(c) >= -D (D + 1) / 2 for c >= -D, and columns up to n + D
+    const size_t slots = (size_t)(nslots + 31) / 32 * 32;
+    // masked neighbours: C(c) >= -D (D + 1) / 2 for c >= -D, and columns up to n + D; what is
+    // there is read and discarded
     const size_t before = sizeof(cplx<R>) * (size_t)(D * (D + 1) / 2 + D + 1);
     const size_t after = sizeof(cplx<R>) * (size_t)(packed_col(n + D + 1, D) + n - packed_col(n, D));
     size_t o = 0;
     L.dd = o;   o = align16(o + sizeof(R) * 6 * ((size_t)n + 1));
-    L.dg = o;   o = align16(o + sizeof(R) * 2 * ((size_t)n + 1));
+    L.dg = o;   o = align16(o + sizeof(R) * ((size_t)n + 1));
     L.sd = o;   o = align16(o + sizeof(R) * 4 * (size_t)n + 32);
-    L.es = o;   o = align16(o + sizeof(double) * 4 * 32);
+    L.es = o;   o = align16(o + sizeof(double) * 4 * 16);
+    L.ell = o;  o = align16(o + sizeof(uint32_t) * ((size_t)n + 1));      // the sites' masks
     L.xs = o;   if (dense_coul) o = align16(o + sizeof(R) * coul_scratch<R>(n));
     if (o < before) o = align16(before);
-    L.x = o;    o = align16(o + sizeof(cplx<R>) * (size_t)packed_col(n, D));
+    L.x = o;    o = align16(o + sizeof(cplx<R>) * (size_t)(packed_col(n - 1, D) + n));
     const size_t x_end = o;
-    L.rho = o;  o = align16(o + sizeof(cplx<R>) * 2 * (size_t)slots);
-    L.lo = o;   if (comp) o = align16(o + sizeof(uint32_t) * 2 * (size_t)slots);
+    L.rho = o;  o = align16(o + sizeof(cplx<R>) * 2 * slots);
+    L.lo = o;   if (comp) o = align16(o + sizeof(uint32_t) * 2 * slots);
     if (o < x_end + after) o = align16(x_end + after);
-    L.ell = L.uv = o;
+    L.uv = o;
     L.total = o;
     return L;
 }
@@ -665,15 +668,20 @@ __device__ __forceinline__ double packed_next(int stage, double rho, double a, d
     return __dadd_rn(rho, __dmul_rn(__dmul_rn(__dadd_rn(b, a), h), 0.125));
 }
 
-template <typename R, int NT, int SPT, int NS>
+// MEMC: the slots' codes are read again for each pass, from the order table (the next one a
+// round ahead) and the sites' masks, instead of held in two registers per slot; that leaves
+// room for 11 slots of RK accumulators, FP32 up to n = 144 (12x12 grid, 512 trajectories x 41
+// steps: 27.2 ms on two CTAs per spin, 15.4 here).
+template <typename R, int NT, int SPT, int NS, bool MEMC = false>
 __global__ void __launch_bounds__(NT, 1) k_pair_packed(ResArgs<R> a)
 {
+    static_assert(NT == 512, "packed_layout has room for 16 warps' energy partials");
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr bool kFloat = std::is_same<R, float>::value;
     const int n = a.sys.n, ne = a.sys.ne, D = a.pat.off[0];
     const int E = a.nslots, DS = n + 1;
     const bool comp = kFloat && a.state64 != nullptr;
-    const ResLayout<R> L = packed_layout<R>(n, NT * SPT, comp, D, a.sys.ud != nullptr);
+    const ResLayout<R> L = packed_layout<R>(n, a.nslots, comp, D, a.sys.ud != nullptr);
     cplx<R>* X = reinterpret_cast<cplx<R>*>(smem + L.x);
     cplx<R>* rhoS = reinterpret_cast<cplx<R>*>(smem + L.rho);
     uint32_t* loS = reinterpret_cast<uint32_t*>(smem + L.lo);
@@ -697,22 +705,40 @@ __global__ void __launch_bounds__(NT, 1) k_pair_packed(ResArgs<R> a)
     bool lost = false;
 
     typename PairAcc<R>::T Ar[2 * SPT], Br[2 * SPT];
-    uint32_t ix[SPT], fl[SPT];
-#pragma unroll
-    for (int q = 0; q < SPT; ++q) {
-        const int f = tid + q * NT;
-        ix[q] = 0u;
-        fl[q] = PAIR_NONE | PAIR_ONE;
-        const uint32_t p = f < E ? a.order[f] : ~0u;
-        if (p == ~0u) continue;
-        const uint32_t i = p & 0xffffu, j = (p >> 16) & 0x7fffu;
+    uint32_t* mk = reinterpret_cast<uint32_t*>(smem + L.ell);
+    for (int j = tid; j <= n; j += NT) mk[j] = j < n ? a.pat.mask[j] : 0u;
+    __syncthreads();
+    struct Slot {
+        int i, j;
+        uint32_t fl;                         // as in k_pair
+    };
+    auto order_at = [&](int f) { return f < E ? __ldg(a.order + f) : ~0u; };
+    auto slot_of = [&](uint32_t p) -> Slot {
+        if (p == ~0u) return Slot{0, 0, PAIR_NONE | PAIR_ONE};
+        const int i = (int)(p & 0xffffu), j = (int)((p >> 16) & 0x7fffu);
         const bool one = (p & PAIR_NONE) != 0;
-        ix[q] = i | (j << 10);
-        fl[q] = a.pat.mask[j] | ((one ? 0u : a.pat.mask[j + 1]) << (2 * NS)) | (a.pat.mask[i] << (4 * NS)) |
-                (one ? PAIR_ONE : 0u);
+        return Slot{i, j, mk[j] | ((one ? 0u : mk[j + 1]) << (2 * NS)) | (mk[i] << (4 * NS)) | (one ? PAIR_ONE : 0u)};
+    };
+    uint32_t ix[MEMC ? 1 : SPT], fl[MEMC ? 1 : SPT];
+    if constexpr (!MEMC) {
+#pragma unroll
+        for (int q = 0; q < SPT; ++q) {
+            const Slot s = slot_of(order_at(tid + q * NT));
+            ix[q] = (uint32_t)s.i | ((uint32_t)s.j << 10);
+            fl[q] = s.fl;
+        }
     }
-    auto i_of = [&](int q) { return (int)(ix[q] & 1023u); };
-    auto j_of = [&](int q) { return (int)(ix[q] >> 10); };
+    // slot q; `next` carries the following one's code (MEMC)
+    auto get = [&](int q, uint32_t& next) -> Slot {
+        if constexpr (MEMC) {
+            const uint32_t p = next;
+            next = order_at(tid + (q + 1) * NT);
+            return slot_of(p);
+        } else {
+            return Slot{(int)(ix[q] & 1023u), (int)(ix[q] >> 10), fl[q]};
+        }
+    };
+    auto first = [&]() -> uint32_t { if constexpr (MEMC) return order_at(tid); else return 0u; };
     for (int q = tid; q < 6 * DS; q += NT) Dd[q] = R(0);
     for (int j = tid; j < n; j += NT) {
         sd[j] = a.sys.tdiag[j];
@@ -720,19 +746,23 @@ __global__ void __launch_bounds__(NT, 1) k_pair_packed(ResArgs<R> a)
         sd[2 * n + j] = a.sys.ediag[j];
         sd[3 * n + j] = a.sys.proj[j];
     }
-    for (int q = tid; q < packed_col(n, D); q += NT) X[q] = cplx<R>{R(0), R(0)};   // rows past n - 1
+    for (int q = tid; q < packed_col(n - 1, D) + n; q += NT) X[q] = cplx<R>{R(0), R(0)};   // rows past n - 1
     double* myslot = a.slots ? a.slots + (size_t)blockIdx.x * a.Tp * W : nullptr;
     cl.sync();
     for (int b = cid; b < a.B; b += ncl) {
         const size_t base = ((size_t)b * 2 + rank) * ne;
+        uint32_t nc = first();
 #pragma unroll
         for (int q = 0; q < SPT; ++q) {
-            const int f = tid + q * NT, i = i_of(q), j = j_of(q);
+            Ar[2 * q] = Br[2 * q] = Ar[2 * q + 1] = Br[2 * q + 1] = {};
+            if ((tid & ~31) + q * NT >= E) continue;
+            const Slot sl = get(q, nc);
+            const int f = tid + q * NT, i = sl.i, j = sl.j;
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 cplx<R> v = {R(0), R(0)};
                 uint32_t lo = 0;
-                if (!(fl[q] & PAIR_NONE) && !(e && (fl[q] & PAIR_ONE))) {
+                if (!(sl.fl & PAIR_NONE) && !(e && (sl.fl & PAIR_ONE))) {
                     const int c = j + e;
                     if (comp) {
                         const cplx<double> x = a.state64[base + cs(c) + i];
@@ -751,7 +781,6 @@ __global__ void __launch_bounds__(NT, 1) k_pair_packed(ResArgs<R> a)
                 }
                 rhoS[2 * f + e] = v;
                 if (comp) loS[2 * f + e] = lo;
-                Ar[2 * q + e] = Br[2 * q + e] = {};
             }
         }
         bool dd_ok = false;                  // Dd[ph] already holds this stage's diagonal
@@ -762,14 +791,17 @@ __global__ void __launch_bounds__(NT, 1) k_pair_packed(ResArgs<R> a)
                 res_record<R, NT, true>(a, [&](int, int k, int j) { return X[packed_col(j, D) + k].re; }, dg,
                                         [&](int) { return od + ph * DS; }, es, myslot + (size_t)t * W, b, rank, tid);
                 if (a.whole) {
+                    uint32_t nc = first();
 #pragma unroll
                     for (int q = 0; q < SPT; ++q) {
-                        if (fl[q] & PAIR_NONE) continue;
-                        const int f = tid + q * NT, i = i_of(q), j = j_of(q);
+                        if ((tid & ~31) + q * NT >= E) break;
+                        const Slot sl = get(q, nc);
+                        if (sl.fl & PAIR_NONE) continue;
+                        const int f = tid + q * NT, i = sl.i, j = sl.j;
                         double2* w = a.whole + ((size_t)t * 2 + rank) * ne;
 #pragma unroll
                         for (int e = 0; e < 2; ++e) {
-                            if (e && (fl[q] & PAIR_ONE)) continue;
+                            if (e && (sl.fl & PAIR_ONE)) continue;
                             atomicAdd(&w[cs(j + e) + i].x, (double)rhoS[2 * f + e].re);
                             atomicAdd(&w[cs(j + e) + i].y, (double)rhoS[2 * f + e].im);
                         }
@@ -795,17 +827,19 @@ __global__ void __launch_bounds__(NT, 1) k_pair_packed(ResArgs<R> a)
                         asm volatile("{\n\t.reg .b64 s;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 s, [%0], %1;\n\t}"
                                      ::"r"(mbar_a + 8 * nph), "r"((uint32_t)(2 * n * (int)sizeof(R))) : "memory");
                     // k of every slot
+                    uint32_t nc = first();
 #pragma unroll
                     for (int q = 0; q < SPT; ++q) {
                         if ((tid & ~31) + q * NT >= E) break;       // this warp's remaining slots are empty
-                        const int i = i_of(q), j = j_of(q);
+                        const Slot sl = get(q, nc);
+                        const int i = sl.i, j = sl.j;
                         const PackedAddr<NS> ad = {j, D, a.pat.off};
                         const int xo = packed_col(j, D) + i;
                         if constexpr (kFloat) {
                             const uint64_t* xp = reinterpret_cast<const uint64_t*>(X) + xo;
                             const uint64_t o0 = xp[0], o1 = xp[ad.next()];
                             uint64_t g0, g1;
-                            pair_sums_f32<NS>(xp, ad, fl[q], a.pat, o0, o1, Dc[i], Dc[j], Dc[j + 1], g0, g1);
+                            pair_sums_f32<NS>(xp, ad, sl.fl, a.pat, o0, o1, Dc[i], Dc[j], Dc[j + 1], g0, g1);
                             if (stage == 0) { Ar[2 * q] = g0; Ar[2 * q + 1] = g1; }
                             else if (stage == 1) { Br[2 * q] = g0; Br[2 * q + 1] = g1; }
                             else if (stage == 2) {
@@ -814,19 +848,21 @@ __global__ void __launch_bounds__(NT, 1) k_pair_packed(ResArgs<R> a)
                             } else { Ar[2 * q] = g0; Ar[2 * q + 1] = g1; }
                         } else {
                             cplx<R> k0, k1;
-                            pair_sums_f64<NS>(X + xo, ad, fl[q], a.pat, Dc[i], Dc[j], Dc[j + 1], k0, k1);
+                            pair_sums_f64<NS>(X + xo, ad, sl.fl, a.pat, Dc[i], Dc[j], Dc[j + 1], k0, k1);
                             packed_acc(stage, k0.re, Ar[2 * q].re, Br[2 * q].re);
                             packed_acc(stage, k0.im, Ar[2 * q].im, Br[2 * q].im);
                             packed_acc(stage, k1.re, Ar[2 * q + 1].re, Br[2 * q + 1].re);
                             packed_acc(stage, k1.im, Ar[2 * q + 1].im, Br[2 * q + 1].im);
                         }
                     }
+                    nc = first();
                     __syncthreads();         // every thread is done reading X
 #pragma unroll
                     for (int q = 0; q < SPT; ++q) {
                         const int f = tid + q * NT;
                         if ((tid & ~31) + q * NT >= E) break;
-                        const int i = i_of(q), j = j_of(q);
+                        const Slot sl = get(q, nc);
+                        const int i = sl.i, j = sl.j;
                         cplx<R> x0, x1;
                         if constexpr (kFloat) {
                             const ulonglong2 rr = reinterpret_cast<const ulonglong2*>(rhoS)[f];
@@ -852,11 +888,11 @@ __global__ void __launch_bounds__(NT, 1) k_pair_packed(ResArgs<R> a)
                             x1.im = packed_next(stage, r1.im, Ar[2 * q + 1].im, Br[2 * q + 1].im, a.h);
                             if (stage == 3) { rhoS[2 * f] = x0; rhoS[2 * f + 1] = x1; }
                         }
-                        if (fl[q] & PAIR_NONE) continue;
+                        if (sl.fl & PAIR_NONE) continue;
                         const int cj = packed_col(j, D), ci = packed_col(i, D);
                         if (j - i <= D) X[ci + j] = cplx<R>{x0.re, -x0.im};
                         X[cj + i] = x0;                       // on the diagonal this second store wins
-                        if (!(fl[q] & PAIR_ONE)) {
+                        if (!(sl.fl & PAIR_ONE)) {
                             if (j + 1 - i <= D) X[ci + j + 1] = cplx<R>{x1.re, -x1.im};
                             X[cj + j + D + 1 + i] = x1;
                         }
@@ -891,13 +927,16 @@ __global__ void __launch_bounds__(NT, 1) k_pair_packed(ResArgs<R> a)
                 }
             }
         }
+        nc = first();
 #pragma unroll
         for (int q = 0; q < SPT; ++q) {
-            if (fl[q] & PAIR_NONE) continue;
-            const int f = tid + q * NT, i = i_of(q), j = j_of(q);
+            if ((tid & ~31) + q * NT >= E) break;
+            const Slot sl = get(q, nc);
+            if (sl.fl & PAIR_NONE) continue;
+            const int f = tid + q * NT, i = sl.i, j = sl.j;
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                if (e && (fl[q] & PAIR_ONE)) continue;
+                if (e && (sl.fl & PAIR_ONE)) continue;
                 const cplx<R> v = rhoS[2 * f + e];
                 const size_t ge = base + cs(j + e) + i;
                 if (comp) {

@@ -111,7 +111,8 @@ const std::vector<VjpCfg<double>>& vjp_cfgs<double>();
     {NT, SPT, SPLIT, {k_pair<R, NT, SPT, SPLIT, 2>, k_pair<R, NT, SPT, SPLIT, 3>},  \
      {k_pair<R, NT, SPT, SPLIT, 2, true>, k_pair<R, NT, SPT, SPLIT, 3, true>}}
 
-#define FPSG_PACKED(R, NT, SPT) {NT, SPT, {k_pair_packed<R, NT, SPT, 2>, k_pair_packed<R, NT, SPT, 3>}, {}, 1}
+#define FPSG_PACKED(R, NT, SPT, MEMC) \
+    {NT, SPT, {k_pair_packed<R, NT, SPT, 2, MEMC>, k_pair_packed<R, NT, SPT, 3, MEMC>}, {}, 1}
 
 #define FPSG_QUAD(R, NT, EPT)                                                                     \
     {NT, EPT, {k_resident_quad<R, NT, EPT, 5>, k_resident_quad<R, NT, EPT, 9>, k_resident_quad<R, NT, EPT, 13>, \
