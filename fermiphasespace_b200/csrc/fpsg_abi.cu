@@ -596,11 +596,16 @@ ResPlan plan_resident(fpsg_ctx* ctx, int B, bool comp = false)
     return plan.idx < 0 ? plan_resident_of<R>(ctx, B, comp, false) : plan;
 }
 
+// One wave of 4-CTA clusters (four SMs per trajectory) ends before one of 2-CTA clusters
+// does (10x10 grid, FP64, 1 trajectory x 400 steps: 10.3 against 13.0 ms), but only a quarter
+// of the SM count of them run at a time.
+bool few_trajectories(const fpsg_ctx* ctx, int B) { return B <= ctx->sm_count / 5; }
+
 // The 4-CTA-cluster kernel for matrices too large for k_resident: the smallest
 // elements-per-thread whose half-matrix slots cover both halves and whose shared
 // memory (the full matrix once, half the element states) fits.
 template <typename R>
-ResPlan plan_quad(fpsg_ctx* ctx, bool comp)
+ResPlan plan_quad(fpsg_ctx* ctx, bool comp, int B)
 {
     ResPlan best;
     const int n = ctx->n, ne = ctx->ne;
@@ -621,6 +626,8 @@ ResPlan plan_quad(fpsg_ctx* ctx, bool comp)
         for (int c = 0; c < (int)hf.size(); ++c) {
             const int nh = hf[c].nh;
             if (nh == 2 && !(std::is_same<R, double>::value || Wc <= 5)) continue;
+            // few FP64 trajectories: four SMs for each (see choose_resident)
+            if (nh == 1 && std::is_same<R, double>::value && few_trajectories(ctx, B)) continue;
             const int cap = hf[c].nt * hf[c].ept;
             if (cap < (nh == 2 ? need : ne)) continue;
             const size_t sm = quad_hp_layout<R>(n, Wc, cap, e8).total;
@@ -674,16 +681,13 @@ ResPlan choose_resident(fpsg_ctx* ctx, int B)
     if (plan.idx < 0 || !plan.pair) {
         const ResPlan pk = plan_packed<R>(ctx, comp_ok);
         if (pk.idx >= 0) plan = pk;
-        // few trajectories: one wave of 4-CTA clusters (four SMs per trajectory) ends before
-        // one of 2-CTA clusters does (10x10 grid, FP64, 1 trajectory x 400 steps: 10.3 against
-        // 13.0 ms), but only a quarter of the SM count of them run at a time
-        if (std::is_same<R, double>::value && pk.idx >= 0 && B <= ctx->sm_count / 5) {
-            const ResPlan two = plan_quad<R>(ctx, false);
-            if (two.idx >= 0 && two.hp) plan = two;
+        if (std::is_same<R, double>::value && pk.idx >= 0 && few_trajectories(ctx, B)) {
+            const ResPlan two = plan_quad<R>(ctx, false, B);
+            if (two.idx >= 0 && two.hp && two.nh == 2) plan = two;
         }
     }
-    if (plan.idx < 0 && comp_ok) plan = plan_quad<R>(ctx, true);
-    if (plan.idx < 0) plan = plan_quad<R>(ctx, false);
+    if (plan.idx < 0 && comp_ok) plan = plan_quad<R>(ctx, true, B);
+    if (plan.idx < 0) plan = plan_quad<R>(ctx, false, B);
     return plan;
 }
 

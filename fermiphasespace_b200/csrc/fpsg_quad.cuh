@@ -517,7 +517,7 @@ __device__ __forceinline__ void quad_hp_pass(int stage, const R* __restrict__ M,
                                              cplx<R> (&Ar)[EPT], cplx<R> (&Br)[EPT], uint32_t (&lo)[EPT], bool comp,
                                              R h, int tid, int n, int P, R* __restrict__ dgn, uint32_t sib_dgn,
                                              bool fuse, uint32_t pDd0, uint32_t pDd1, const R* __restrict__ sd,
-                                             const DevSys<R>& sys, R pvn)
+                                             const DevSys<R>& sys, R pvn, int half)
 {
     // FP64 sums the diagonal terms in place (the oracle's order); FP32 drops them from
     // the sums and adds X_ij (Delta_jj - Delta_ii) afterwards (no cancellation)
@@ -525,6 +525,9 @@ __device__ __forceinline__ void quad_hp_pass(int stage, const R* __restrict__ M,
 #pragma unroll
     for (int q = 0; q < EPT; ++q) {
         const int f = tid + q * NT;
+        // this warp's remaining slots are empty (they would cost as much as real ones: fcc, 32
+        // sites, FP32, 2048 trajectories x 42 steps: 91 ms with all 12 rounds)
+        if ((NH == 2 ? quad_slot(f & ~31, half) : (f & ~31)) >= sys.ne) break;
         const bool valid = ix[q] != ~0u;
         const int i = valid ? (int)(ix[q] & 1023u) : 0;
         const int j = valid ? (int)((ix[q] >> 10) & 1023u) : 0;
@@ -640,7 +643,7 @@ __device__ __forceinline__ void quad_hp_pass(int stage, const R* __restrict__ M,
 // trajectory, one CTA per spin holding all of its elements: no sibling, and every SM
 // usable, where the spin's state fits beside the two matrix buffers).
 template <typename R, int NT, int EPT, int W, bool E8, int NH>
-__global__ void __launch_bounds__(NT, 1) k_resident_quad_hp(ResArgs<R> a)
+__global__ void __launch_bounds__(NT, NT <= 256 ? 512 / NT : 1) k_resident_quad_hp(ResArgs<R> a)
 {
     static_assert(NH == 1 || NH == 2, "one or two CTAs per spin");
     static_assert(E8 || sizeof(Ent<R>) == 16, "FP32 column entries are the 8-byte kind");
@@ -816,7 +819,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident_quad_hp(ResArgs<R> a)
             for (int st = 0; st < nsteps; ++st, ++gstep) {
 #define FPSG_HP_PASS(S_)                                                                                   \
     quad_hp_pass<R, NT, EPT, S_, W, E8, NH>(stage, Mr, Mw, sMw, ell, Ddc, rhoS, ix, Ar, Br, lo, comp, a.h, tid, n, P, \
-                                        dgw, sdgw, fuse, pd0, pd1, sd, a.sys, pvn)
+                                        dgw, sdgw, fuse, pd0, pd1, sd, a.sys, pvn, half)
 #define FPSG_HP_STAGE_BODY                                                                                     \
                     const int nxt = cur ^ 1;                                                                          \
                     R* Ddc = Dd + cur * n;                                                                            \

@@ -119,11 +119,11 @@ const std::vector<VjpCfg<double>>& vjp_cfgs<double>();
                k_resident_quad<R, NT, EPT, 17>}, {}}
 
 // FP64: 16-byte (FP64 weights) and 8-byte (FP32-exact weights) column entries
-#define FPSG_QUAD_HP64(NT, EPT)                                                                         \
-    {NT, EPT, {k_resident_quad_hp<double, NT, EPT, 5, false, 2>, k_resident_quad_hp<double, NT, EPT, 9, false, 2>, \
-               k_resident_quad_hp<double, NT, EPT, 13, false, 2>, k_resident_quad_hp<double, NT, EPT, 17, false, 2>}, \
-              {k_resident_quad_hp<double, NT, EPT, 5, true, 2>, k_resident_quad_hp<double, NT, EPT, 9, true, 2>,     \
-               k_resident_quad_hp<double, NT, EPT, 13, true, 2>, k_resident_quad_hp<double, NT, EPT, 17, true, 2>}}
+#define FPSG_QUAD_HP64(NT, EPT, NH_)                                                                    \
+    {NT, EPT, {k_resident_quad_hp<double, NT, EPT, 5, false, NH_>, k_resident_quad_hp<double, NT, EPT, 9, false, NH_>, \
+               k_resident_quad_hp<double, NT, EPT, 13, false, NH_>, k_resident_quad_hp<double, NT, EPT, 17, false, NH_>}, \
+              {k_resident_quad_hp<double, NT, EPT, 5, true, NH_>, k_resident_quad_hp<double, NT, EPT, 9, true, NH_>,     \
+               k_resident_quad_hp<double, NT, EPT, 13, true, NH_>, k_resident_quad_hp<double, NT, EPT, 17, true, NH_>}, NH_}
 // FP32: 8-byte entries only; NH_ CTAs per spin (2: 4-CTA clusters, 1: 2-CTA clusters)
 #define FPSG_QUAD_HP32(NT, EPT, NH_)                                                                    \
     {NT, EPT, {k_resident_quad_hp<float, NT, EPT, 5, true, NH_>, k_resident_quad_hp<float, NT, EPT, 9, true, NH_>,   \
