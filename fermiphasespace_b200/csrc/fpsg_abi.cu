@@ -572,7 +572,10 @@ ResPlan plan_resident_of(fpsg_ctx* ctx, int B, bool comp, bool pair)
         const double elem_fill = (double)(M * items) / cap;                       // thread utilisation
         const double row_fill = (double)(M * n) / (32.0 * ((M * n + 31) / 32));     // lane utilisation
         const double split_pen = cf[c].split ? 0.9 : 1.0;
-        const double score = elem_fill * row_fill * split_pen - 0.002 * cf[c].ept * (pair ? 2 : 1);
+        double score = elem_fill * row_fill * split_pen - 0.002 * cf[c].ept * (pair ? 2 : 1);
+        // one trajectory (Hartree-Fock): nothing else fills the GPU, so a stage's latency counts,
+        // which is its rounds of one item per thread
+        if (B == 1) score = -(double)((M * items + cf[c].nt - 1) / cf[c].nt) - (cf[c].split ? 0.5 : 0.0);
         if (score > best_score) {
             best_score = score;
             best.idx = c; best.G = G;
@@ -1197,14 +1200,15 @@ int dense_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
     };
     auto cleanup = [&]() { for (void* p : temps) trelease(ctx, p); };
     const size_t mat = (size_t)M * 2 * NP * NP;
-    float *R = nullptr, *Xa = nullptr, *Xb = nullptr, *Xc = nullptr, *Tf = nullptr, *Ud = nullptr, *Vd = nullptr;
+    float *R = nullptr, *Xa = nullptr, *Xb = nullptr, *Xc = nullptr, *Tf = nullptr, *Ud = nullptr, *Vd = nullptr,
+          *dvec = nullptr;
     void* Tc = nullptr;
     const bool tf32 = q.precision == FPSG_PREC_SPLIT_TF32X3;
     unsigned* d_err = nullptr;
     if ((rc = tmp((void**)&R, sizeof(float) * mat)) || (rc = tmp((void**)&Xa, sizeof(float) * mat)) ||
         (rc = tmp((void**)&Xb, sizeof(float) * mat)) || (rc = tmp((void**)&Xc, sizeof(float) * mat)) ||
         (rc = tmp((void**)&Tf, sizeof(float) * NP * NP)) ||
-        (rc = tmp(&Tc, TC_BYTES)) ||
+        (rc = tmp(&Tc, TC_BYTES)) || (rc = tmp((void**)&dvec, sizeof(float) * (size_t)M * NP)) ||
         (rc = tmp((void**)&d_err, sizeof(unsigned)))) {
         cleanup();
         return rc;
@@ -1273,7 +1277,7 @@ int dense_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
     const int grid = std::max(1, std::min(M, ctx->sm_count));
 
     DenseArgs da;
-    da.n = n; da.M = M; da.Tc = Tc; da.sys = sys; da.err = d_err; da.Ud = Ud; da.Vd = Vd;
+    da.n = n; da.M = M; da.Tc = Tc; da.sys = sys; da.err = d_err; da.Ud = Ud; da.Vd = Vd; da.dvec = dvec;
     // test hook: the call's first launch waits on a barrier nothing arrives at
     da.probe_polls = (ctx->flags & FPSG_FLAG_TEST_EXPIRE_WAIT) ? 4096u : 0u;
     double tc = q.record ? 0.0 : q.t_start;
@@ -1289,7 +1293,7 @@ int dense_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
             }
             CK(launch_stage(da, grid, tf32, ctx->stream));
             da.probe_polls = 0;
-            out.launches++;
+            out.launches += 2;
         }
         tc += h;
         return FPSG_OK;

@@ -21,7 +21,7 @@
 //
 // One launch = one RK stage of every spin matrix.  Persistent CTAs (one per SM),
 // warp-specialised:
-//   warps 0-15  epilogue: Hartree diagonal d of the matrix, then per plane read
+//   warps 0-15  epilogue: per plane read
 //               the accumulator from tensor memory and write
 //               out = a0 P0 + a1 P1 + ax X + hk k (the 3/8 RK rule in terms of
 //               stored stage inputs)
@@ -68,8 +68,7 @@ __host__ __device__ __forceinline__ int canon(int r, int k)
 struct Shared {
     // after the stage buffers
     float d[2][NP];          // Delta_jj of the matrix (double-buffered by matrix)
-    float nd[2][NP];         // diagonals: other spin, same spin
-    uint64_t fullX[STAGES];  // producers' conversions done (128 arrivals)
+    uint64_t fullX[STAGES];  // producers' conversions done (an arrival per warp)
     uint64_t fullT[STAGES];  // T bulk copies landed (1 arrival + bytes)
     uint64_t empty[STAGES];  // MMAs reading the stage are done
     uint64_t tfull[2];       // accumulator tile mt complete
@@ -131,6 +130,34 @@ __device__ __forceinline__ void split4_tf32(const float4& u, uint4& big, uint4& 
     small = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
+// The planes of the epilogue's block EPI_AHEAD blocks on (possibly of the next tile, plane
+// or matrix) into L2, 1 KB per plane and warp.  The epilogue holds one block's loads in
+// registers and has no room for a second; from DRAM a block took 3.4 to 4.8 K cycles, and
+// the epilogue was busy for 95 % of the kernel (1150 -> 991 us per stage, 2048 matrices).
+constexpr int EPI_AHEAD = 4;
+__device__ __forceinline__ void epi_prefetch(const DenseArgs& a, int m, int p, int mt, int q4, int hh, int jb)
+{
+    constexpr int NB = EPI_COLS / EPI_BLK;
+    if (jb >= NB) {
+        jb -= NB;
+        if (++mt == 2) {
+            mt = 0;
+            if (++p == 2) {
+                p = 0;
+                m += gridDim.x;
+                if (m >= a.M) return;
+            }
+        }
+    }
+    const size_t off = (size_t)m * 2 * PLANE + plane_off(mt * 128 + q4 * 32, hh * EPI_COLS + jb * EPI_BLK);
+    const size_t op = off + (size_t)p * PLANE, oq = off + (size_t)(1 - p) * PLANE;
+    constexpr uint32_t bytes = 32 * EPI_BLK * sizeof(float);       // 32 rows x EPI_BLK columns: contiguous
+    tc::prefetch_l2(a.X + op, bytes);
+    tc::prefetch_l2(a.X + oq, bytes);
+    if (a.P0) tc::prefetch_l2(a.P0 + oq, bytes);
+    if (a.P1) tc::prefetch_l2(a.P1 + oq, bytes);
+}
+
 template <bool TF32>
 __global__ void __launch_bounds__(NTHREADS, 1) k_dense_stage(DenseArgs a)
 {
@@ -146,7 +173,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_dense_stage(DenseArgs a)
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
-            tc::mbar_init(&sh->fullX[s], N_PROD_WARPS * 32);
+            tc::mbar_init(&sh->fullX[s], N_PROD_WARPS);
             tc::mbar_init(&sh->fullT[s], 1);
             tc::mbar_init(&sh->empty[s], 1);
         }
@@ -190,7 +217,23 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_dense_stage(DenseArgs a)
                 const float* Xp = a.X + (size_t)m * mstride + (size_t)(pm >> 1) * PLANE;
                 for (int kc = 0; kc < NCHE; ++kc, ++it) {
                     const int s = it % STAGES;
-                    if (!wait_bar(&sh->empty[s], ((it / STAGES) & 1) ^ 1, sh, a.err)) { ok = false; break; }
+                    // the chunk two on into L2: 8 row blocks of KCE columns, contiguous each
+                    if (pw == 0 && lane < NP / 32 && kc + 2 < NCHE)
+                        tc::prefetch_l2(Xp + plane_off(lane * 32, (kc + 2) * KCE), 32 * KCE * sizeof(float));
+                    // the loads go out before the stage is free
+                    // lane (r8, kq): one 16-byte core row of row r, K-core kq
+                    float4 v[NP / 8 / N_PROD_WARPS][TF32 ? 1 : 2];
+#pragma unroll
+                    for (int q = 0; q < NP / 8 / N_PROD_WARPS; ++q) {
+                        const int r = (pw + q * N_PROD_WARPS) * 8 + r8;
+                        const int k = kc * KCE + kq * EPC;
+                        v[q][0] = __ldg(reinterpret_cast<const float4*>(Xp + plane_off(r, k)));
+                        if constexpr (!TF32) v[q][TF32 ? 0 : 1] = __ldg(reinterpret_cast<const float4*>(Xp + plane_off(r, k + 4)));
+                    }
+                    // one lane polls; the outcome is the warp's
+                    uint32_t got = 1;
+                    if (lane == 0) got = wait_bar(&sh->empty[s], ((it / STAGES) & 1) ^ 1, sh, a.err) ? 1u : 0u;
+                    if (!__shfl_sync(0xffffffffu, got, 0)) { ok = false; break; }
                     unsigned char* st = stages + (size_t)s * STAGE_BYTES;
                     if (pt == 0) {
                         const char* tcb = reinterpret_cast<const char*>(a.Tc);
@@ -202,15 +245,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_dense_stage(DenseArgs a)
                     }
                     T* xh = reinterpret_cast<T*>(st);
                     T* xl = xh + TILE_E;
-                    // lane (r8, kq): one 16-byte core row of row r, K-core kq
-                    float4 v[NP / 8 / N_PROD_WARPS][TF32 ? 1 : 2];
-#pragma unroll
-                    for (int q = 0; q < NP / 8 / N_PROD_WARPS; ++q) {
-                        const int r = (pw + q * N_PROD_WARPS) * 8 + r8;
-                        const int k = kc * KCE + kq * EPC;
-                        v[q][0] = __ldg(reinterpret_cast<const float4*>(Xp + plane_off(r, k)));
-                        if constexpr (!TF32) v[q][TF32 ? 0 : 1] = __ldg(reinterpret_cast<const float4*>(Xp + plane_off(r, k + 4)));
-                    }
 #pragma unroll
                     for (int q = 0; q < NP / 8 / N_PROD_WARPS; ++q) {
                         const int r = (pw + q * N_PROD_WARPS) * 8 + r8;
@@ -221,7 +255,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_dense_stage(DenseArgs a)
                         *reinterpret_cast<uint4*>(xl + canon<EPC>(r, kq * EPC)) = lo;
                     }
                     tc::fence_async_smem();
-                    tc::mbar_arrive(&sh->fullX[s]);
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&sh->fullX[s]);
                 }
             }
         }
@@ -295,47 +330,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_dense_stage(DenseArgs a)
         // ------------------------------------------------------------ epilogue
         const int et = threadIdx.x;                 // 0 .. 32 N_EPI_WARPS - 1
         const int q4 = warp & 3, hh = warp >> 2;
-        const DevSys<float>& sy = a.sys;
         int ue[2] = {0, 0}, mi = 0;              // uses of each accumulator tile
         bool ok = true;
         for (int m = blockIdx.x; m < a.M && ok; m += gridDim.x, ++mi) {
             const float* Xm = a.X + (size_t)m * mstride;
-            const float* Xo = a.X + (size_t)(m ^ 1) * mstride;
-            // Delta_jj = ((tM_jj + sum U (n_other + s)) + sum V (n_same + s)) + ext_jj + pulse proj_j
-            for (int j = et; j < NP; j += N_EPI_WARPS * 32) {
-                sh->nd[0][j] = j < a.n ? Xo[plane_off(j, j)] : 0.f;
-                sh->nd[1][j] = j < a.n ? Xm[plane_off(j, j)] : 0.f;
-            }
-            tc::named_sync(1, N_EPI_WARPS * 32);
-            for (int j = et; j < NP; j += N_EPI_WARPS * 32) {
-                float dj = 0.f;
-                if (j < a.n) {
-                    dj = sy.tdiag[j];
-                    if (a.Ud) {
-                        // long-range Coulomb: U and V are symmetric, so thread j walks
-                        // column j and the warp reads each row k contiguously
-                        float uacc = 0.f, vacc = 0.f;
-                        for (int k = 0; k < a.n; ++k) uacc += a.Ud[(size_t)k * NP + j] * (sh->nd[0][k] + sy.shift);
-                        dj += uacc;
-                        if (sy.coul == 2) {
-                            for (int k = 0; k < a.n; ++k) vacc += a.Vd[(size_t)k * NP + j] * (sh->nd[1][k] + sy.shift);
-                            dj += vacc;
-                        }
-                    } else if (sy.coul != 0) {
-                        float uacc = 0.f;
-                        for (int q = sy.up[j]; q < sy.up[j + 1]; ++q) uacc += sy.uv[q] * (sh->nd[0][sy.uk[q]] + sy.shift);
-                        dj += uacc;
-                        if (sy.coul == 2) {
-                            float vacc = 0.f;
-                            for (int q = sy.vp[j]; q < sy.vp[j + 1]; ++q) vacc += sy.vv[q] * (sh->nd[1][sy.vk[q]] + sy.shift);
-                            dj += vacc;
-                        }
-                    }
-                    if (sy.has_ext) dj += sy.ediag[j];
-                    if (sy.n_bins > 0) dj += a.pulse * sy.proj[j];
-                }
-                sh->d[mi & 1][j] = dj;
-            }
+            for (int j = et; j < NP; j += N_EPI_WARPS * 32) sh->d[mi & 1][j] = __ldg(a.dvec + (size_t)m * NP + j);
             tc::named_sync(1, N_EPI_WARPS * 32);
             const float* dd = sh->d[mi & 1];
             for (int p = 0; p < 2 && ok; ++p) {
@@ -360,6 +359,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_dense_stage(DenseArgs a)
 #pragma unroll 1
                     for (int jb = 0; jb < EPI_COLS / EPI_BLK; ++jb) {
                         const int j0 = hh * EPI_COLS + jb * EPI_BLK;
+                        if (lane == 0) epi_prefetch(a, m, p, mt, q4, hh, jb + EPI_AHEAD);
                         // global loads first: their latency overlaps the tensor-memory read
                         const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
                         float4 vp[EPI_BLK / 4], vq[EPI_BLK / 4], v0[EPI_BLK / 4], v1[EPI_BLK / 4];
@@ -404,6 +404,59 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_dense_stage(DenseArgs a)
     if (warp == MMA_WARP) {
         tc::tc_fence_after();
         tc::tmem_dealloc(tbase, TMEM_COLS);
+    }
+}
+
+// Delta_jj = ((tM_jj + sum U (n_other + s)) + sum V (n_same + s)) + ext_jj + pulse proj_j of
+// every matrix, DIAG_T trajectories per CTA: one read of row k of U and V serves their 2
+// DIAG_T matrices.  Inside the stage kernel the same sums were one thread's chain of 2 n
+// loads per site before the matrix's epilogue could begin: half of the kernel's time at
+// n = 256 (1440 -> 1150 us per stage and 2048 matrices, and 70 us here).
+constexpr int DIAG_T = 4;
+__global__ void __launch_bounds__(NP) k_dense_diag(DenseArgs a)
+{
+    __shared__ float nd[2 * DIAG_T][NP];                 // n_jj + shift by matrix
+    const DevSys<float>& sy = a.sys;
+    const int j = threadIdx.x, m0 = 2 * DIAG_T * blockIdx.x, nm = min(2 * DIAG_T, a.M - m0);
+#pragma unroll
+    for (int q = 0; q < 2 * DIAG_T; ++q)
+        nd[q][j] = (q < nm && j < a.n) ? a.X[(size_t)(m0 + q) * 2 * PLANE + plane_off(j, j)] + sy.shift : 0.f;
+    __syncthreads();
+    float u[2 * DIAG_T], v[2 * DIAG_T];
+#pragma unroll
+    for (int q = 0; q < 2 * DIAG_T; ++q) u[q] = v[q] = 0.f;
+    if (a.Ud) {
+        // U and V are symmetric: thread j walks column j, the warp reads row k
+#pragma unroll 8
+        for (int k = 0; k < a.n; ++k) {
+            const float uk = __ldg(a.Ud + (size_t)k * NP + j), vk = __ldg(a.Vd + (size_t)k * NP + j);
+#pragma unroll
+            for (int q = 0; q < 2 * DIAG_T; ++q) {
+                u[q] = fmaf(uk, nd[q ^ 1][k], u[q]);
+                v[q] = fmaf(vk, nd[q][k], v[q]);
+            }
+        }
+    } else if (sy.coul != 0 && j < a.n) {
+        for (int x = sy.up[j]; x < sy.up[j + 1]; ++x)
+#pragma unroll
+            for (int q = 0; q < 2 * DIAG_T; ++q) u[q] = fmaf(sy.uv[x], nd[q ^ 1][sy.uk[x]], u[q]);
+        if (sy.coul == 2)
+            for (int x = sy.vp[j]; x < sy.vp[j + 1]; ++x)
+#pragma unroll
+                for (int q = 0; q < 2 * DIAG_T; ++q) v[q] = fmaf(sy.vv[x], nd[q][sy.vk[x]], v[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < 2 * DIAG_T; ++q) {
+        if (q >= nm) continue;
+        float d = 0.f;
+        if (j < a.n) {
+            d = sy.tdiag[j];
+            if (sy.coul != 0) d += u[q];
+            if (sy.coul == 2) d += v[q];
+            if (sy.has_ext) d += sy.ediag[j];
+            if (sy.n_bins > 0) d += a.pulse * sy.proj[j];
+        }
+        a.dvec[(size_t)(m0 + q) * NP + j] = d;
     }
 }
 
@@ -572,6 +625,7 @@ cudaError_t configure()
 
 cudaError_t launch_stage(const DenseArgs& a, int grid, bool tf32, cudaStream_t st)
 {
+    k_dense_diag<<<(a.M + 2 * DIAG_T - 1) / (2 * DIAG_T), NP, 0, st>>>(a);
     if (tf32) k_dense_stage<true><<<grid, NTHREADS, stage_smem_bytes(), st>>>(a);
     else k_dense_stage<false><<<grid, NTHREADS, stage_smem_bytes(), st>>>(a);
     return cudaGetLastError();

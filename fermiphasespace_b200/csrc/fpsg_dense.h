@@ -43,6 +43,7 @@ struct DenseArgs {
     DevSys<float> sys;           // diagonal terms (tM_jj, Hartree rows, potential, pulse projection)
     const float* Ud;             // dense U, V ([NP][NP], zero-padded) for long-range Coulomb, else null
     const float* Vd;
+    float* dvec;                 // [M][NP] Delta_jj of the stage input (k_dense_diag)
     float pulse;                 // pulse amplitude x envelope at the stage time
     unsigned* err;
     // test hook (FPSG_FLAG_TEST_EXPIRE_WAIT): > 0 makes one thread wait, with this

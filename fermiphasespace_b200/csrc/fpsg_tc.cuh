@@ -57,6 +57,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
     return false;
 }
 
+// Brings `bytes` (a multiple of 16) of global memory at a 16-byte aligned address into L2,
+// without waiting and without a destination in shared memory.
+__device__ __forceinline__ void prefetch_l2(const void* g, uint32_t bytes)
+{
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(g), "r"(bytes) : "memory");
+}
+
 // ---------------------------------------------------------------- bulk copy
 // Global -> this CTA's shared memory, completion counted on `bar` in bytes.
 // Both addresses 16-byte aligned, size a multiple of 16.
