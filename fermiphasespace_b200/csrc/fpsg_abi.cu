@@ -559,8 +559,8 @@ ResPlan plan_resident_of(fpsg_ctx* ctx, int B, bool comp, bool pair)
         const int per = cf[c].split ? 1 : 2;
         const int cap = cf[c].nt * cf[c].ept;
         auto bytes = [&](int G, bool uv = false) {
-            return pair ? pair_layout<R>(n, per * G, cap, comp, t.pat.off[0], t.ud != nullptr, uv).total
-                        : res_layout_direct<R>(n, per * G, t.ell_p, cap, comp, t.ud != nullptr).total;
+            return pair ? pair_layout<R>(n, per * G, cap, comp, t.pat.off[0], t.ud != nullptr, uv, cf[c].split).total
+                        : res_layout_direct<R>(n, per * G, t.ell_p, cap, comp, t.ud != nullptr, cf[c].split).total;
         };
         int Gmax = std::min(cap / (per * items), PAIR_MMAX / per);
         while (Gmax > 0 && bytes(Gmax) > ctx->smem_optin) --Gmax;
@@ -678,17 +678,20 @@ template <typename R>
 ResPlan choose_resident(fpsg_ctx* ctx, int B)
 {
     const bool comp_ok = !std::is_same<R, double>::value && !(ctx->flags & FPSG_FLAG_FP32_PLAIN_STATE);
-    ResPlan plan;
-    if (comp_ok) plan = plan_resident<R>(ctx, B, true);
-    if (plan.idx < 0) plan = plan_resident<R>(ctx, B);
+    ResPlan plan = plan_resident<R>(ctx, B, comp_ok);
+    // k_pair_packed where k_pair does not fit, before anything without the compensated update
     if (plan.idx < 0 || !plan.pair) {
         const ResPlan pk = plan_packed<R>(ctx, comp_ok);
-        if (pk.idx >= 0) plan = pk;
-        if (std::is_same<R, double>::value && pk.idx >= 0 && few_trajectories(ctx, B)) {
-            const ResPlan two = plan_quad<R>(ctx, false, B);
-            if (two.idx >= 0 && two.hp && two.nh == 2) plan = two;
+        if (pk.idx >= 0) {
+            plan = pk;
+            if (std::is_same<R, double>::value && few_trajectories(ctx, B)) {
+                const ResPlan two = plan_quad<R>(ctx, false, B);
+                if (two.idx >= 0 && two.hp && two.nh == 2) plan = two;
+            }
+            return plan;
         }
     }
+    if (plan.idx < 0 && comp_ok) plan = plan_resident<R>(ctx, B);
     if (plan.idx < 0 && comp_ok) plan = plan_quad<R>(ctx, true, B);
     if (plan.idx < 0) plan = plan_quad<R>(ctx, false, B);
     return plan;
@@ -1421,9 +1424,16 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
         const size_t traj = sizeof(cplx<R>) * 2 * (size_t)ne;
         const size_t per_keep = traj * 4 * (size_t)C * (size_t)nseg;          // every segment kept
         const size_t per_tmp = traj * (size_t)(10 + nck + 4 * C);              // the chunk's scratch
-        size_t fre = 0, tot = 0, pooled = 0;
-        if (cudaMemGetInfo(&fre, &tot) != cudaSuccess) { cudaGetLastError(); fre = 0; }
-        for (const auto& a : ctx->pool) pooled += a.bytes;
+        size_t fre = 0, tot = 0, pooled = 0, largest = 0;
+        for (const auto& a : ctx->pool) {
+            pooled += a.bytes;
+            largest = std::max(largest, a.bytes);
+        }
+        // A pooled buffer that holds every stage input of the whole ensemble (a previous call of
+        // this shape left it) needs no look at the free memory, a driver call that has been seen
+        // to take tens of milliseconds on a busy host.
+        const bool fits = largest >= (size_t)Ball * per_keep;
+        if (!fits && cudaMemGetInfo(&fre, &tot) != cudaSuccess) { cudaGetLastError(); fre = 0; }
         size_t avail = fre + pooled;       // pooled scratch is reused or released
         if (ctx->mem_cap) {
             const size_t held = ctx->mem_used > pooled ? ctx->mem_used - pooled : 0;
@@ -1432,7 +1442,7 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
         const size_t budget = avail / 4 * 3;
         long nchunk = 1;
         const size_t need = (size_t)Ball * (per_keep + per_tmp);
-        if (budget > 0 && need > budget) nchunk = (long)((need + budget - 1) / budget);
+        if (!fits && budget > 0 && need > budget) nchunk = (long)((need + budget - 1) / budget);
         if (ctx->grad_keep > 0)
             nchunk = std::max<long>(nchunk, (long)(((size_t)Ball * per_keep + (size_t)ctx->grad_keep - 1) / (size_t)ctx->grad_keep));
         nchunk = std::min<long>(nchunk, Ball / ctx->sm_count);
@@ -1576,8 +1586,8 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
                     budget = std::min<size_t>(budget, ctx->mem_cap > ctx->mem_used ? (ctx->mem_cap - ctx->mem_used) / 4 * 3 : 0);
                 return std::min<long>(want, (long)(budget / segbytes));
             };
-            long fresh = fresh_segments();
             const long pooled = bi >= 0 ? std::min<long>(want, (long)(ctx->pool[bi].bytes / segbytes)) : 0;
+            long fresh = pooled > 0 && pooled >= want ? 0 : fresh_segments();
             if (pooled > 0 && pooled >= fresh) {
                 keep = (cplx<R>*)ctx->pool[bi].p;
                 n_keep = (int)pooled;

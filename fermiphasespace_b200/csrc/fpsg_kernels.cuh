@@ -578,10 +578,11 @@ __device__ __forceinline__ R delta_diag_v(const DevSys<R>& s, int j, const R* sa
 // 14 K of the 24 K cycles of a stage at 63 sites, FP32, both spins in the CTA; this takes
 // 3 K.
 template <typename R>
-__host__ __device__ __forceinline__ size_t coul_scratch(int RR)
+__host__ __device__ __forceinline__ size_t coul_scratch(int RR, bool both)
 {
-    const size_t two = 2 * (size_t)RR;
-    return std::is_same<R, float>::value && two < 1024 ? 1024 : two;
+    if (!std::is_same<R, float>::value) return 2 * (size_t)RR;
+    const size_t threads = both ? 1024 : 512;            // a partial sum (both: two) per thread
+    return (size_t)RR > threads ? (size_t)RR : threads;
 }
 template <typename R, int NT, bool BOTH, typename SAME, typename OTHER>
 __device__ __forceinline__ void delta_diag_block(const DevSys<R>& s, const R* ud, const R* vd, R* Dc, R* scr, int RR,
@@ -778,7 +779,7 @@ __device__ __forceinline__ void res_record(const ResArgs<R>& a, RE re, const R* 
 // double-buffered: the pass reads X[cur] and writes X[cur ^ 1].
 template <typename R>
 __host__ __device__ __forceinline__ ResLayout<R> res_layout_direct(int n, int M, int P, int nt_ept, bool comp = false,
-                                                                   bool dense_coul = false)
+                                                                   bool dense_coul = false, bool split = false)
 {
     ResLayout<R> L;
     const size_t RP = (size_t)((M * n) | 1);
@@ -790,7 +791,7 @@ __host__ __device__ __forceinline__ ResLayout<R> res_layout_direct(int n, int M,
     L.es = o;   o = align16(o + sizeof(double) * 4 * 32);               // energy partials per warp
     L.ell = o;  o = align16(o + sizeof(Ent<R>) * (size_t)n * (2 * P + 1));
     L.lo = o;   if (comp) o = align16(o + sizeof(uint32_t) * (size_t)nt_ept);   // bf16 residual pairs
-    L.xs = o;   if (dense_coul) o = align16(o + sizeof(R) * coul_scratch<R>(M * n));
+    L.xs = o;   if (dense_coul) o = align16(o + sizeof(R) * coul_scratch<R>(M * n, !split));
     L.total = o;
     return L;
 }
@@ -948,7 +949,7 @@ __global__ void __launch_bounds__(NT, 1) k_resident(ResArgs<R> a)
     const int SPARE = n * RP;
     constexpr int NE = 2 * P + 1;
     const bool comp = std::is_same<R, float>::value && a.state64 != nullptr;
-    const ResLayout<R> L = res_layout_direct<R>(n, M, P, NT * EPT, comp, a.sys.ud != nullptr);
+    const ResLayout<R> L = res_layout_direct<R>(n, M, P, NT * EPT, comp, a.sys.ud != nullptr, SPLIT);
     uint32_t* loS = comp ? reinterpret_cast<uint32_t*>(smem + L.lo) : nullptr;
     cplx<R>* Xb = reinterpret_cast<cplx<R>*>(smem + L.x);
     cplx<R>* rhoS = reinterpret_cast<cplx<R>*>(smem + L.rho);

@@ -66,7 +66,7 @@ inline std::vector<uint32_t> pair_slot_order(int n)
 
 template <typename R>
 __host__ __device__ __forceinline__ ResLayout<R> pair_layout(int n, int M, int slots, bool comp, int max_off,
-                                                             bool dense_coul, bool coul_smem)
+                                                             bool dense_coul, bool coul_smem, bool split)
 {
     ResLayout<R> L;
     const size_t RP = (size_t)((M * n) | 1);
@@ -83,7 +83,7 @@ __host__ __device__ __forceinline__ ResLayout<R> pair_layout(int n, int M, int s
     L.sd = o;   o = align16(o + sizeof(R) * 4 * (size_t)n + 32);          // tM_jj, U_jj, extPot_jj, pulse; 3 mbarriers
     L.es = o;   o = align16(o + sizeof(double) * 4 * 32);
     L.lo = o;   if (comp) o = align16(o + sizeof(uint32_t) * 2 * (size_t)slots);
-    L.xs = o;   if (dense_coul) o = align16(o + sizeof(R) * coul_scratch<R>(M * n));
+    L.xs = o;   if (dense_coul) o = align16(o + sizeof(R) * coul_scratch<R>(M * n, !split));
     L.uv = o;   if (coul_smem) o = align16(o + sizeof(R) * 2 * (size_t)n * n);
     if (o < x_end + guard) o = align16(x_end + guard);
     L.ell = o;
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_pair(ResArgs<R> a)
     const int XS = n * RP;
     const bool comp = std::is_same<R, float>::value && a.state64 != nullptr;
     const ResLayout<R> L = pair_layout<R>(n, M, NT * SPT, comp, a.pat.off[0], a.sys.ud != nullptr,
-                                             a.coul_smem != 0);
+                                             a.coul_smem != 0, SPLIT);
     uint32_t* loS = comp ? reinterpret_cast<uint32_t*>(smem + L.lo) : nullptr;
     cplx<R>* Xb = reinterpret_cast<cplx<R>*>(smem + L.x);
     cplx<R>* rhoS = reinterpret_cast<cplx<R>*>(smem + L.rho);
@@ -605,17 +605,30 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_pair(ResArgs<R> a)
 // 10x10 grid, FP64, 4096 trajectories x 41 steps: 134.7 -> 77.0 ms
 __host__ __device__ __forceinline__ int packed_col(int c, int D) { return (c * (c + 2 * D + 1)) >> 1; }
 
+// C(j + o) - C(j) = o j + up[s], C(j - o) - C(j) = dn[s] - o j for the offsets o of a
+// pattern, and from column j + 1 the column's length more
+template <int NS>
+struct PackedOffs {
+    int o[NS], up[NS], dn[NS];
+    __device__ __forceinline__ PackedOffs(const int (&off)[PAT_MAX], int D)
+    {
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            o[s] = s == NS - 1 ? 1 : off[s];
+            up[s] = (o[s] * (o[s] + 2 * D + 1)) >> 1;
+            dn[s] = (o[s] * (o[s] - 2 * D - 1)) >> 1;
+        }
+    }
+};
 template <int NS>
 struct PackedAddr {
     int j, D;
-    const int (&off)[PAT_MAX];
+    const PackedOffs<NS>& k;
     __device__ __forceinline__ int next() const { return j + D + 1; }
-    // C(j + e + sgn off) - C(j), from C(c + o) - C(c) = o c + o (o + 2 D + 1) / 2
     __device__ __forceinline__ int col(int s, int sgn, int e) const
     {
-        const int o = s == NS - 1 ? 1 : off[s];
-        const int d = sgn * o + e;
-        return d * j + ((d * (d + 2 * D + 1)) >> 1);
+        const int o = k.o[s], c = sgn > 0 ? o * j + k.up[s] : k.dn[s] - o * j;
+        return e ? c + j + sgn * o + D + 1 : c;
     }
 };
 
@@ -634,7 +647,7 @@ __host__ __device__ __forceinline__ ResLayout<R> packed_layout(int n, int nslots
     L.sd = o;   o = align16(o + sizeof(R) * 4 * (size_t)n + 32);
     L.es = o;   o = align16(o + sizeof(double) * 4 * 16);
     L.ell = o;  o = align16(o + sizeof(uint32_t) * ((size_t)n + 1));      // the sites' masks
-    L.xs = o;   if (dense_coul) o = align16(o + sizeof(R) * coul_scratch<R>(n));
+    L.xs = o;   if (dense_coul) o = align16(o + sizeof(R) * coul_scratch<R>(n, false));
     if (o < before) o = align16(before);
     L.x = o;    o = align16(o + sizeof(cplx<R>) * (size_t)(packed_col(n - 1, D) + n));
     const size_t x_end = o;
@@ -703,6 +716,7 @@ __global__ void __launch_bounds__(NT, 1) k_pair_packed(ResArgs<R> a)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     uint32_t ph = 0, parity = 0;
     bool lost = false;
+    const PackedOffs<NS> offs(a.pat.off, D);
 
     typename PairAcc<R>::T Ar[2 * SPT], Br[2 * SPT];
     uint32_t* mk = reinterpret_cast<uint32_t*>(smem + L.ell);
@@ -833,7 +847,7 @@ __global__ void __launch_bounds__(NT, 1) k_pair_packed(ResArgs<R> a)
                         if ((tid & ~31) + q * NT >= E) break;       // this warp's remaining slots are empty
                         const Slot sl = get(q, nc);
                         const int i = sl.i, j = sl.j;
-                        const PackedAddr<NS> ad = {j, D, a.pat.off};
+                        const PackedAddr<NS> ad = {j, D, offs};
                         const int xo = packed_col(j, D) + i;
                         if constexpr (kFloat) {
                             const uint64_t* xp = reinterpret_cast<const uint64_t*>(X) + xo;
