@@ -1013,7 +1013,7 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
         // With an offset pattern the pair stage, where a matrix has work for its 512 threads: it
         // takes 0.3 ms per stage against 0.7 (n = 256, FP32, 512 trajectories), and in shared
         // memory too k_stream_stage is the slower one (n = 143, FP64, 300 trajectories: 0.51
-        // against 0.25 ms).
+        // against 0.16 ms).
         const DevTables<R>& tb = tables<R>(ctx);
         const bool sp = !fock && tb.pat_ns != 0 && (gx || ctx->n_pair >= 2 * SP_NT);
         auto sp_fn = tb.pat_ns == 3 ? k_stream_pair<R, 3> : k_stream_pair<R, 2>;
@@ -1632,7 +1632,7 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
     // the segment-resident reverse kernel: on-site (or no) Coulomb term, an offset pattern or
     // fixed-width columns with P <= 4, the packed matrix within the slots of a configuration;
     // the smallest one that holds it (5x5 grid, FP64, 300 trajectories, ten steps: 545 us with
-    // 512 threads per CTA, 128 with 128)
+    // 512 threads per CTA, 300 with 128)
     const DevTables<R>& tv = tables<R>(ctx);
     const int seg_v = tv.pat_ns && n < 256 ? tv.pat_ns : ellP == 2 ? 0 : 1;
     const VjpCfg<R>* seg_cfg = nullptr;

@@ -528,7 +528,7 @@ __global__ void k_dense_pack(const float* __restrict__ X, int n, int M, cplx<R>*
 // potential rows as one sweep of each spin's real plane against tM in the same order (16-byte
 // loads, FP64 sums), the Coulomb rows from dense U and V with the threads along a row.  The
 // packed copy and the one-thread-per-site index lists it replaces took 1.76 ms per snapshot
-// at n = 256, 1024 trajectories; this takes 0.25 ms.
+// at n = 256, 1024 trajectories; this takes 0.28 ms.
 constexpr int REC_NT = 256;
 __global__ void __launch_bounds__(REC_NT) k_dense_record(DenseRecordArgs a)
 {

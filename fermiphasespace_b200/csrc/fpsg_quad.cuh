@@ -517,7 +517,7 @@ __device__ __forceinline__ void quad_hp_pass(int stage, const R* __restrict__ M,
                                              cplx<R> (&Ar)[EPT], cplx<R> (&Br)[EPT], uint32_t (&lo)[EPT], bool comp,
                                              R h, int tid, int n, int P, R* __restrict__ dgn, uint32_t sib_dgn,
                                              bool fuse, uint32_t pDd0, uint32_t pDd1, const R* __restrict__ sd,
-                                             const DevSys<R>& sys, R pvn, int half)
+                                             const DevSys<R>& sys, R pvn, int nq)
 {
     // FP64 sums the diagonal terms in place (the oracle's order); FP32 drops them from
     // the sums and adds X_ij (Delta_jj - Delta_ii) afterwards (no cancellation)
@@ -526,8 +526,9 @@ __device__ __forceinline__ void quad_hp_pass(int stage, const R* __restrict__ M,
     for (int q = 0; q < EPT; ++q) {
         const int f = tid + q * NT;
         // this warp's remaining slots are empty (they would cost as much as real ones: fcc, 32
-        // sites, FP32, 2048 trajectories x 42 steps: 91 ms with all 12 rounds)
-        if ((NH == 2 ? quad_slot(f & ~31, half) : (f & ~31)) >= sys.ne) break;
+        // sites, FP32, 2048 trajectories x 42 steps: 91 ms with all 12 rounds).  With two CTAs
+        // per spin the configurations are fitted instead: the test costs 3 % in full rounds.
+        if (NH == 1 && q >= nq) break;
         const bool valid = ix[q] != ~0u;
         const int i = valid ? (int)(ix[q] & 1023u) : 0;
         const int j = valid ? (int)((ix[q] >> 10) & 1023u) : 0;
@@ -707,6 +708,8 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 512 / NT : 1) k_resident_quad_
         sd[2 * n + j] = a.sys.ediag[j];
         sd[3 * n + j] = a.sys.proj[j];
     }
+    int nq = 0;                                     // rounds in which this warp has elements (NH = 1)
+    while (nq < EPT && (tid & ~31) + nq * NT < ne) ++nq;
     double* myslot = a.slots ? a.slots + (size_t)blockIdx.x * a.Tp * RW : nullptr;
     // padding entries (weight 0) read rows < n only; the spare words take no reads
     for (int q = tid; q < 2 * MW; q += NT) M[q] = R(0);
@@ -819,7 +822,7 @@ __global__ void __launch_bounds__(NT, NT <= 256 ? 512 / NT : 1) k_resident_quad_
             for (int st = 0; st < nsteps; ++st, ++gstep) {
 #define FPSG_HP_PASS(S_)                                                                                   \
     quad_hp_pass<R, NT, EPT, S_, W, E8, NH>(stage, Mr, Mw, sMw, ell, Ddc, rhoS, ix, Ar, Br, lo, comp, a.h, tid, n, P, \
-                                        dgw, sdgw, fuse, pd0, pd1, sd, a.sys, pvn, half)
+                                        dgw, sdgw, fuse, pd0, pd1, sd, a.sys, pvn, nq)
 #define FPSG_HP_STAGE_BODY                                                                                     \
                     const int nxt = cur ^ 1;                                                                          \
                     R* Ddc = Dd + cur * n;                                                                            \
