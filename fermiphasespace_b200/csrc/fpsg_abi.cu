@@ -528,6 +528,18 @@ double host_pulse(const fpsg_ctx* c, double t)
 }
 
 // ------------------------------------------------------------------ resident configs
+// The limit belongs to the function, not to a launch: set to one plan's size, it would be
+// too small for the launch of another context, or of another system of a batch, whose
+// setup came before.  So it is always the most that the device gives the kernel.
+cudaError_t allow_smem(const fpsg_ctx* ctx, const void* fn, size_t smem)
+{
+    cudaFuncAttributes fa;
+    const cudaError_t e = cudaFuncGetAttributes(&fa, fn);
+    if (e != cudaSuccess) return e;
+    const size_t most = ctx->smem_optin > fa.sharedSizeBytes ? ctx->smem_optin - fa.sharedSizeBytes : 0;
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(most, smem));
+}
+
 static int p_index(int P) { return P == 2 ? 0 : P == 4 ? 1 : 2; }
 
 struct ResPlan {
@@ -741,7 +753,7 @@ struct ResLauncher {
             const QuadCfg<R>& qc = (plan.pair ? packed_cfgs<R>() : plan.hp ? quad_hp_cfgs<R>() : quad_cfgs<R>())[plan.idx];
             fn = (plan.hp && plan.e8 ? qc.fn8 : qc.fn)[plan.pair ? tables<R>(ctx).pat_ns - 2 : quad_w_index(tables<R>(ctx).cell_w)];
             nt = qc.nt; split = false; cdim = plan.hp || plan.pair ? 2 * plan.nh : 4; smem = plan.smem;
-            CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CK(allow_smem(ctx, (const void*)fn, smem));
             cudaLaunchConfig_t lc = config(ctx, cdim * B);
             cudaLaunchAttribute at[1];
             cluster_attr(at, lc);
@@ -755,7 +767,7 @@ struct ResLauncher {
         const int v = plan.pair ? tables<R>(ctx).pat_ns - 2 : p_index(tables<R>(ctx).ell_p);
         fn = dump ? cfg.fn_dump[v] : cfg.fn[v];
         nt = cfg.nt; split = cfg.split; cdim = split ? 2 : 1; smem = plan.smem;
-        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(allow_smem(ctx, (const void*)fn, smem));
         const int ngroups = (B + plan.G - 1) / plan.G;
         if (split) {
             cudaLaunchConfig_t lc = config(ctx, 2 * ngroups);
@@ -829,7 +841,7 @@ struct FockLauncher {
         smem = fock_layout<R>(ctx->n, d_smem, tv_smem).total;
         if (smem > ctx->smem_optin) return false;
         fn = tv_smem ? k_fock_run<R, true, true> : d_smem ? k_fock_run<R, true, false> : k_fock_run<R, false, false>;
-        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        if (allow_smem(ctx, (const void*)fn, smem) != cudaSuccess ||
             cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
             cudaGetLastError();
             return false;
@@ -1006,7 +1018,7 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
         const bool gx = smem > ctx->smem_optin;
         if (gx) smem = ((sizeof(R) * n + 15) & ~size_t(15)) + sizeof(double) * 32 * 4;
         auto stage_fn = gx ? k_stream_stage<R, true> : k_stream_stage<R, false>;
-        CK(cudaFuncSetAttribute(stage_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(allow_smem(ctx, (const void*)stage_fn, smem));
         int per_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stage_fn, 256, smem));
         const int grid = std::max(1, std::min(2 * B, std::max(1, per_sm) * ctx->sm_count));
@@ -1020,7 +1032,7 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
         const size_t sp_smem = stream_pair_smem(n, sizeof(R));
         int sp_grid = 1;
         if (sp) {
-            CK(cudaFuncSetAttribute(sp_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp_smem));
+            CK(allow_smem(ctx, (const void*)sp_fn, sp_smem));
             int occ = 0;
             CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sp_fn, SP_NT, sp_smem));
             sp_grid = std::max(1, std::min(2 * B, std::max(1, occ) * ctx->sm_count));
@@ -1501,8 +1513,8 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
     const size_t smem = ((sizeof(cplx<R>) * ne + sizeof(R) * n + 15) & ~size_t(15)) + sizeof(double) * 32 * 4;
     const size_t vsmem = ((2 * sizeof(cplx<R>) * ne + 2 * sizeof(R) * n + 15) & ~size_t(15)) + sizeof(double) * 32 * 3;
     if (smem > ctx->smem_optin || vsmem > ctx->smem_optin) { cleanup(); return fail(ctx, FPSG_ERR_UNSUPPORTED, "system too large for the adjoint kernels"); }
-    CK(cudaFuncSetAttribute(k_stream_stage<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CK(cudaFuncSetAttribute(k_vjp_stage<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vsmem));
+    CK(allow_smem(ctx, (const void*)k_stream_stage<R>, smem));
+    CK(allow_smem(ctx, (const void*)k_vjp_stage<R>, vsmem));
     int per_sm = 0, vper_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stream_stage<R>, 256, smem));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&vper_sm, k_vjp_stage<R>, 256, vsmem));
@@ -1623,7 +1635,7 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
     auto ell_fn = ellP == 2 ? k_vjp_stage_ell<R, 2> : ellP == 4 ? k_vjp_stage_ell<R, 4> : k_vjp_stage_ell<R, 8>;
     int egrid = 1;
     if (use_ell) {
-        CK(cudaFuncSetAttribute(ell_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)esmem));
+        CK(allow_smem(ctx, (const void*)ell_fn, esmem));
         int per_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ell_fn, 256, esmem));
         egrid = std::max(1, std::min(2 * B, std::max(1, per_sm) * ctx->sm_count));
@@ -1666,7 +1678,7 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
         auto clusters = [&](ResKernelVjp<R> fn, size_t sm, int& ncl) -> int {
             ncl = 0;
             if (sm > ctx->smem_optin) return FPSG_OK;
-            CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+            CK(allow_smem(ctx, (const void*)fn, sm));
             cudaLaunchConfig_t lc = {};
             lc.gridDim = dim3(2 * B); lc.blockDim = dim3(SEG_NT); lc.dynamicSmemBytes = sm; lc.stream = ctx->stream;
             lc.attrs = at; lc.numAttrs = 1;
@@ -2085,6 +2097,7 @@ int batch_impl(fpsg_ctx* ctx, const fpsg_system_desc* sd, int ns, int method, do
                     cudaGraph_t g = nullptr;
                     cudaStreamEndCapture(ctx->stream, &g);
                     if (g) cudaGraphDestroy(g);
+                    cudaGetLastError();          // the ended capture's error is not the next call's
                     const std::string why = c->err;
                     cleanup();
                     return fail(ctx, FPSG_ERR_CUDA, why);
@@ -2150,7 +2163,7 @@ int batch_impl(fpsg_ctx* ctx, const fpsg_system_desc* sd, int ns, int method, do
     double tune_ms = 0.0;
     std::vector<StreamArgs<R>> ha;
     if (nss > 0) {
-        CK(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(allow_smem(ctx, (const void*)kfn, smem));
         // stage arguments: variant 0 = stage 0 recording a snapshot, 1..4 = stages 0..3
         ha.resize((size_t)5 * nss);
         for (int v = 0; v < 5; ++v)
@@ -2684,7 +2697,7 @@ int fpsg_gpsr_drift(fpsg_ctx* ctx, int B, const double* rho, double t, double d_
     const size_t smem = gpsr_smem_bytes(n, a.stage_x_in_smem != 0);
     void (*fns[4])(GpsrArgs) = {k_gpsr_stage<0>, k_gpsr_stage<1>, k_gpsr_stage<2>, k_gpsr_stage<3>};
     int per_sm = 1;
-    for (auto fn : fns) CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    for (auto fn : fns) CK(allow_smem(ctx, (const void*)fn, smem));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fns[0], 256, smem));
     const int grid = std::max(1, std::min(2 * B, std::max(1, per_sm) * ctx->sm_count));
     const cplx<double>* in[4] = {r, x0, x1, x0};

@@ -117,3 +117,27 @@ def compare_fp32(T, coulomb, ext, B):
     state = eng.get_state()
     eng.close()
     return ref, {E.PREC_FP32: (r, state)}
+
+
+@pytest.mark.parametrize("prec,sizes", [(0, [(10, 10), (9, 10), (9, 9)]), (1, [(10, 10), (9, 10), (9, 9)]),
+                                        (1, [(12, 12), (11, 11), (11, 10)]), (0, [(5, 4), (4, 4), (3, 3)])])
+def test_batch_members_of_one_configuration(prec, sizes):
+    # systems of falling size that take the same kernel: the shared memory that the last one
+    # needs must not be the limit of the first one's launch
+    eng = E.Engine()
+    desc = []
+    for k, (nx, ny) in enumerate(sizes):
+        pos = cf.grid_positions(nx, ny, 1)
+        n = nx * ny
+        occ = (np.arange(n) % 2).astype(float)
+        desc.append({"tM": cf.hopping(cf.distances(pos), [(1.0, -1.0)]), "U": 4.0 * np.eye(n), "V": None, "ext": None,
+                     "coulomb": E.COUL_ONSITE, "n_traj": 9, "seed": 5 + k, "occ_up": occ, "occ_dn": 1.0 - occ})
+    res, _ = eng.run_batch(desc, E.METHOD_FTWA, prec, 0.01, 1, 3, obs=1 | 2 | 4 | 16)
+    for d, r in zip(desc, res):
+        eng.set_system(d["tM"], d["U"], None, None, coulomb=E.COUL_ONSITE)
+        eng.sample(9, d["seed"], d["occ_up"], d["occ_dn"])
+        one = eng.run(E.METHOD_FTWA, prec, 0.01, 1, 3, obs=1 | 2 | 4 | 16)
+        assert r.path_used == one.path_used == E.PATH_RESIDENT
+        for key in ("niiu", "niid", "n2iiu", "n2iid", "nund"):
+            assert np.array_equal(getattr(r, key), getattr(one, key)), key
+    eng.close()
