@@ -81,22 +81,33 @@ __device__ __forceinline__ void st_peer(uint32_t a, cplx<float> v)
 
 // Complex numbers from shared memory by 32-bit address: whole (lanes reading consecutive
 // ones), or by component for addresses all lanes share (an 8-byte broadcast is one
-// wavefront, a 16-byte one four).  `epoch` changes with the contents: it keeps the compiler
-// from taking two loads of one address for the same value.
-__device__ __forceinline__ void lds_cplx(cplx<double>& v, uint32_t a, int epoch)
+// wavefront, a 16-byte one four).  The loads are asm that the compiler may move (as volatile
+// ones each waited for the one before: 12 to 21 K cycles for a sweep over k of 7 to 10), so
+// what orders them is data: every address derives from a base taken by after_barrier behind
+// the barrier that publishes the contents, and before_barrier takes what was formed from them
+// ahead of the barrier that lets the contents change.
+__device__ __forceinline__ uint32_t after_barrier(const void* p)
 {
-    asm("ld.shared.v2.f64 {%0, %1}, [%2]; // %3" : "=d"(v.re), "=d"(v.im) : "r"(a), "r"(epoch));
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile("" : "+r"(a)::"memory");
+    return a;
 }
-__device__ __forceinline__ void lds_cplx(cplx<float>& v, uint32_t a, int epoch)
+__device__ __forceinline__ void before_barrier(cplx<double>& v) { asm volatile("" : "+d"(v.re), "+d"(v.im)::"memory"); }
+__device__ __forceinline__ void before_barrier(cplx<float>& v) { asm volatile("" : "+f"(v.re), "+f"(v.im)::"memory"); }
+__device__ __forceinline__ void lds_cplx(cplx<double>& v, uint32_t a)
 {
-    asm("ld.shared.v2.f32 {%0, %1}, [%2]; // %3" : "=f"(v.re), "=f"(v.im) : "r"(a), "r"(epoch));
+    asm("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.re), "=d"(v.im) : "r"(a));
 }
-__device__ __forceinline__ void lds_parts(cplx<double>& v, uint32_t a, int epoch)
+__device__ __forceinline__ void lds_cplx(cplx<float>& v, uint32_t a)
 {
-    asm("ld.shared.f64 %0, [%1]; // %2" : "=d"(v.re) : "r"(a), "r"(epoch));
-    asm("ld.shared.f64 %0, [%1+8]; // %2" : "=d"(v.im) : "r"(a), "r"(epoch));
+    asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.re), "=f"(v.im) : "r"(a));
 }
-__device__ __forceinline__ void lds_parts(cplx<float>& v, uint32_t a, int epoch) { lds_cplx(v, a, epoch); }
+__device__ __forceinline__ void lds_parts(cplx<double>& v, uint32_t a)
+{
+    asm("ld.shared.f64 %0, [%1];" : "=d"(v.re) : "r"(a));
+    asm("ld.shared.f64 %0, [%1+8];" : "=d"(v.im) : "r"(a));
+}
+__device__ __forceinline__ void lds_parts(cplx<float>& v, uint32_t a) { lds_cplx(v, a); }
 
 // DSMEM: Delta in shared memory; TVSMEM: tM, V and the elements' indices too
 template <typename R, bool DSMEM, bool TVSMEM>
@@ -267,20 +278,19 @@ __global__ void __launch_bounds__(FOCK_NT, 1) k_fock_run(FockRunArgs<R> a)
                         // run: a CTA has one or two busy warps per scheduler
                         if constexpr (DSMEM) {
                             const uint32_t sz = (uint32_t)sizeof(cplx<R>), row = (uint32_t)P * sz;
-                            const uint32_t Xa = (uint32_t)__cvta_generic_to_shared(X), Da = (uint32_t)__cvta_generic_to_shared(Dm);
+                            const uint32_t Xa = after_barrier(X), Da = after_barrier(Dm);
                             uint32_t xi = Xa + i * sz, ei = Da + i * sz;
                             uint32_t yj = Xa + j * row, yk = Xa + j1 * row, dj = Da + j * row, dk = Da + j1 * row;
-                            const int ep = (int)g;
                             cplx<R> x, e, d0, d1, y0, y1;
-                            lds_cplx(x, xi, ep); lds_cplx(e, ei, ep);
-                            lds_parts(d0, dj, ep); lds_parts(d1, dk, ep); lds_parts(y0, yj, ep); lds_parts(y1, yk, ep);
+                            lds_cplx(x, xi); lds_cplx(e, ei);
+                            lds_parts(d0, dj); lds_parts(d1, dk); lds_parts(y0, yj); lds_parts(y1, yk);
 #pragma unroll 4
                             for (int k = 1; k < n; ++k) {
                                 xi += row; ei += row;
                                 const cplx<R> cx = x, ce = e, c0 = d0, c1 = d1, v0 = y0, v1 = y1;
-                                lds_cplx(x, xi, ep); lds_cplx(e, ei, ep);
-                                lds_parts(d0, dj + k * sz, ep); lds_parts(d1, dk + k * sz, ep);
-                                lds_parts(y0, yj + k * sz, ep); lds_parts(y1, yk + k * sz, ep);
+                                lds_cplx(x, xi); lds_cplx(e, ei);
+                                lds_parts(d0, dj + k * sz); lds_parts(d1, dk + k * sz);
+                                lds_parts(y0, yj + k * sz); lds_parts(y1, yk + k * sz);
                                 cmaddR<R>(a0.re, a0.im, cx, c0);
                                 cmaddR<R>(a1.re, a1.im, cx, c1);
                                 cmaddR<R>(b0.re, b0.im, v0, ce);
@@ -290,6 +300,7 @@ __global__ void __launch_bounds__(FOCK_NT, 1) k_fock_run(FockRunArgs<R> a)
                             cmaddR<R>(a1.re, a1.im, x, d1);
                             cmaddR<R>(b0.re, b0.im, y0, e);
                             cmaddR<R>(b1.re, b1.im, y1, e);
+                            before_barrier(a0); before_barrier(a1); before_barrier(b0); before_barrier(b1);
                         } else {
                             auto ld = [](const cplx<R>* p) -> cplx<R> {     // written by other SMs: not from L1
                                 using V = typename std::conditional<sizeof(R) == 8, double2, float2>::type;
