@@ -128,6 +128,11 @@ int cuda_fail(fpsg_ctx* c, cudaError_t e, const char* where)
         if (e_ != cudaSuccess) return cuda_fail(ctx, e_, #call);  \
     } while (0)
 
+struct AtExit {
+    std::function<void()> f;
+    ~AtExit() { f(); }
+};
+
 int dalloc(fpsg_ctx* ctx, void** p, size_t bytes)
 {
     *p = nullptr;
@@ -875,7 +880,13 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
         if (!r) temps.push_back(*p);
         return r;
     };
-    auto cleanup = [&]() { for (void* p : temps) trelease(ctx, p); };
+    auto cleanup = [&]() { for (void* p : temps) trelease(ctx, p); temps.clear(); };
+    // a return on a CUDA error gives the scratch back too, once nothing in flight writes it
+    AtExit guard{[&]() {
+        if (temps.empty()) return;
+        cudaStreamSynchronize(ctx->stream);
+        cleanup();
+    }};
 
     const int do_e1 = hf ? (ctx->coul != FPSG_COULOMB_NULL) : 1;
     const int do_e2 = hf ? (ctx->coul == FPSG_COULOMB_DISTANCE) : 1;
@@ -1080,12 +1091,13 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
             fr.diagbuf = nullptr; fr.ebuf = nullptr; fr.whole = whole; fr.order = ctx->pair_order;
             fr.nslots = ctx->n_pair; fr.err = d_err;
             double* fpart = nullptr;
+            const int slab = std::min(q.Tp, 65535);      // snapshots per reduction: the limit of gridDim.y
             const size_t eb = sizeof(double) * (size_t)q.Tp * B * 2 * 4;
             if (!fl.d_smem && (rc = tmp((void**)&fr.Dg, sizeof(cplx<R>) * (size_t)2 * B * n * (n | 1)))) { cleanup(); return rc; }
             if (q.record) {
                 if ((rc = tmp((void**)&fr.diagbuf, sizeof(double) * (size_t)q.Tp * B * 2 * n)) ||
                     (rc = tmp((void**)&fr.ebuf, eb)) ||
-                    (rc = tmp((void**)&fpart, sizeof(double) * (size_t)q.Tp * nch * W))) {
+                    (rc = tmp((void**)&fpart, sizeof(double) * (size_t)slab * nch * W))) {
                     cleanup(); return rc;
                 }
                 CK(cudaMemsetAsync(fr.ebuf, 0, eb, ctx->stream));
@@ -1104,9 +1116,11 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
                 out.launches++;
                 for (int t = t0; t < fr.t_end; ++t) done += (q.record && t == q.Tp - 1) ? 0 : fr.S;
             }
-            if (q.record) {
-                k_reduce_part<<<dim3(nch, q.Tp, (W + 255) / 256), 256, 0, ctx->stream>>>(fr.diagbuf, fr.ebuf, B, n, chunk, fpart);
-                k_reduce_fin<<<dim3(std::max(1, (W + 255) / 256), q.Tp), 256, 0, ctx->stream>>>(fpart, nch, W, sums);
+            for (int t0 = 0; q.record && t0 < q.Tp; t0 += slab) {
+                const int m = std::min(slab, q.Tp - t0);
+                k_reduce_part<<<dim3(nch, m, (W + 255) / 256), 256, 0, ctx->stream>>>(
+                    fr.diagbuf + (size_t)t0 * B * 2 * n, fr.ebuf + (size_t)t0 * B * 2 * 4, B, n, chunk, fpart);
+                k_reduce_fin<<<dim3(std::max(1, (W + 255) / 256), m), 256, 0, ctx->stream>>>(fpart, nch, W, sums + (size_t)t0 * W);
                 CK(cudaGetLastError());
                 out.launches += 2;
             }

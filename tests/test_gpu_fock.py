@@ -49,3 +49,42 @@ def test_fock_matches_oracle(dims, B, S, Tp):
     bound = S * (Tp - 1) * (4 * 0.1 * 4 * np.sqrt(n) + 4) * 2.0 ** -24 * 4
     assert np.max(np.abs(r32.niiu - ref["niiu"])) < bound
     eng.close()
+
+
+def small_system(n, seed=5):
+    rng = np.random.default_rng(seed)
+    D = np.abs(np.arange(n)[:, None] - np.arange(n)[None, :]).astype(float)
+    T = -1.0 * (D == 1)
+    U = 2.0 / (1.0 + D)
+    return T, U, U - np.diag(np.diag(U)), np.diag(rng.uniform(-1, 1, n)), rng
+
+
+def hf_states(T, B, rng):
+    """Projectors on half of the eigenstates of the hopping in random potentials."""
+    n = T.shape[0]
+    rho = np.zeros((B, 2, n, n), dtype=complex)
+    for b in range(B):
+        for s in range(2):
+            R = np.linalg.eigh(T + np.diag(rng.uniform(-1, 1, n)))[1][:, : (n + 1 - s) // 2]
+            rho[b, s] = R @ R.T
+    return (rho + np.conj(np.swapaxes(rho, 2, 3))) / 2
+
+
+def test_fock_more_snapshots_than_a_grid_dimension():
+    """65 538 snapshots, recorded by many launches and reduced in more than one go."""
+    T, U, V, ext, rng = small_system(2)
+    Tp, dt = 65538, 1e-3
+    rho = hf_states(T, 1, rng)
+    pulse = {"n_bins": 3, "amp": rng.normal(0, 0.5, 3), "bin_width": 30.0, "t0": 30.0, "td": 20.0, "proj": np.array([-0.5, 0.5])}
+    ref = orc.run(orc.System(T, U, V, ext, orc.COUL_DISTANCE, False, pulse), 1, dt, 1, Tp, rho, nthreads=1)
+    eng = E.Engine()
+    eng.set_system(T, U, V, ext, E.COUL_DISTANCE)
+    eng.set_pulse(pulse["amp"], pulse["bin_width"], pulse["t0"], pulse["td"], pulse["proj"])
+    eng.set_initial_samples(rho)
+    r = eng.run(E.METHOD_HF, E.PREC_FP64, dt, 1, Tp)
+    assert np.array_equal(eng.get_state(), ref["final"])
+    for k in ("niiu", "niid", "n2iiu", "n2iid", "nund"):
+        assert np.array_equal(getattr(r, k), ref[k]), k
+    # sums of n^2 terms of order 1 in another order
+    assert np.max(np.abs(r.energies - ref["energies"])) < 4 * 4 * 2.0 ** -52 * np.abs(ref["energies"]).max()
+    eng.close()
