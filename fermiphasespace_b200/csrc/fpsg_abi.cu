@@ -1075,8 +1075,24 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
             fa.tMf = dt_; fa.Uf = du_; fa.Vf = dv_; fa.extf = de_; fa.D = dd_;
         }
         FockLauncher<R> fl;
-        if (fock && ((size_t)q.Tp * B * 2 * (n + 4) * sizeof(double) >> 30) == 0 && fl.setup(ctx, B)) {
-            FockRunArgs<R> fr;
+        bool fock_run = fock && ((size_t)q.Tp * B * 2 * (n + 4) * sizeof(double) >> 30) == 0 && fl.setup(ctx, B);
+        FockRunArgs<R> fr;
+        fr.Dg = nullptr; fr.diagbuf = nullptr; fr.ebuf = nullptr;
+        double* fpart = nullptr;
+        const int slab = std::min(q.Tp, 65535);          // snapshots per reduction: the limit of gridDim.y
+        const size_t eb = sizeof(double) * (size_t)q.Tp * B * 2 * 4;
+        if (fock_run) {
+            const size_t held = temps.size();
+            if ((!fl.d_smem && tmp((void**)&fr.Dg, sizeof(cplx<R>) * (size_t)2 * B * n * (n | 1))) ||
+                (q.record && (tmp((void**)&fr.diagbuf, sizeof(double) * (size_t)q.Tp * B * 2 * n) ||
+                              tmp((void**)&fr.ebuf, eb) || tmp((void**)&fpart, sizeof(double) * (size_t)slab * nch * W)))) {
+                // no room for the records of all snapshots: k_fock_stage needs those of one
+                for (; temps.size() > held; temps.pop_back()) trelease(ctx, temps.back());
+                ctx->err.clear();
+                fock_run = false;
+            }
+        }
+        if (fock_run) {
             fr.sys = sys; fr.tMf = fa.tMf; fr.Uf = fa.Uf; fr.Vf = fa.Vf; fr.extf = fa.extf;
             fr.uv_same = fr.ext_diag = 1;
             for (int j = 0; j < n; ++j)
@@ -1085,23 +1101,11 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
                     if (i != j && (R)ctx->U[x] != (R)ctx->V[x]) fr.uv_same = 0;
                     if (i != j && !ctx->ext_null && (R)ctx->ext[x] != R(0)) fr.ext_diag = 0;
                 }
-            fr.state = st; fr.Dg = nullptr; fr.B = B; fr.cps = fl.cps; fr.h = (R)h; fr.hf = q.record;
+            fr.state = st; fr.B = B; fr.cps = fl.cps; fr.h = (R)h; fr.hf = q.record;
             fr.S = q.record ? q.S : 1; fr.Tp = q.record ? q.Tp : 1 << 30;
             fr.record = q.record; fr.do_en = rec_e; fr.do_e1 = do_e1 && rec_e; fr.do_e2 = do_e2 && rec_e;
-            fr.diagbuf = nullptr; fr.ebuf = nullptr; fr.whole = whole; fr.order = ctx->pair_order;
-            fr.nslots = ctx->n_pair; fr.err = d_err;
-            double* fpart = nullptr;
-            const int slab = std::min(q.Tp, 65535);      // snapshots per reduction: the limit of gridDim.y
-            const size_t eb = sizeof(double) * (size_t)q.Tp * B * 2 * 4;
-            if (!fl.d_smem && (rc = tmp((void**)&fr.Dg, sizeof(cplx<R>) * (size_t)2 * B * n * (n | 1)))) { cleanup(); return rc; }
-            if (q.record) {
-                if ((rc = tmp((void**)&fr.diagbuf, sizeof(double) * (size_t)q.Tp * B * 2 * n)) ||
-                    (rc = tmp((void**)&fr.ebuf, eb)) ||
-                    (rc = tmp((void**)&fpart, sizeof(double) * (size_t)slab * nch * W))) {
-                    cleanup(); return rc;
-                }
-                CK(cudaMemsetAsync(fr.ebuf, 0, eb, ctx->stream));
-            }
+            fr.whole = whole; fr.order = ctx->pair_order; fr.nslots = ctx->n_pair; fr.err = d_err;
+            if (q.record) CK(cudaMemsetAsync(fr.ebuf, 0, eb, ctx->stream));
             cudaLaunchAttribute at[1];
             const cudaLaunchConfig_t lc = fl.config(ctx, fl.ncl, at);
             // time chunks, so that one launch stays in the tens of milliseconds

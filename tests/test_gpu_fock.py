@@ -88,3 +88,23 @@ def test_fock_more_snapshots_than_a_grid_dimension():
     # sums of n^2 terms of order 1 in another order
     assert np.max(np.abs(r.energies - ref["energies"])) < 4 * 4 * 2.0 ** -52 * np.abs(ref["energies"]).max()
     eng.close()
+
+
+def test_fock_without_room_for_all_records():
+    """Under a memory cap that holds one snapshot's records but not all of them, the run is the
+    per-stage kernel's."""
+    T, U, V, ext, rng = small_system(3)
+    Tp = 4001
+    rho = hf_states(T, 2, rng)
+    ref = orc.run(orc.System(T, U, V, ext, orc.COUL_DISTANCE, False), 1, 0.005, 1, Tp, rho)
+    eng = E.Engine()
+    eng.set_system(T, U, V, ext, E.COUL_DISTANCE)
+    eng.set_initial_samples(rho)
+    # the sums of all snapshots take 19 doubles each; with every record there are 19 + 2 (3 + 4) 2 more
+    eng.set_memory_cap(8 * Tp * 19 + (1 << 18))
+    r = eng.run(E.METHOD_HF, E.PREC_FP64, 0.005, 1, Tp)
+    assert np.array_equal(eng.get_state(), ref["final"])
+    # the mean of two trajectories, each value exact: the order of the sum does not matter
+    for k in ("niiu", "niid", "n2iiu", "n2iid", "nund"):
+        assert np.array_equal(getattr(r, k), ref[k]), k
+    eng.close()
