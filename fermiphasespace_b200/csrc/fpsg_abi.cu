@@ -820,7 +820,7 @@ struct ResLauncher {
 // The cluster kernel of HF with the Fock term (fpsg_fock.cuh): the widest cluster the
 // device takes (16 CTAs, 8 per spin; else 8) whose slots cover the matrix, with X (and
 // Delta, where it fits too) in shared memory: n <= 84 in FP64 with both, n <= 119 with X
-// alone.  Larger systems run k_fock_stage.
+// alone.  Larger systems run k_fock_stage, and so do ensembles that it is faster for.
 template <typename R>
 struct FockLauncher {
     void (*fn)(FockRunArgs<R>) = nullptr;
@@ -858,9 +858,27 @@ struct FockLauncher {
             const cudaLaunchConfig_t lc = config(ctx, B, at);
             if (cudaOccupancyMaxActiveClusters(&ncl, (void*)fn, &lc) != cudaSuccess) { cudaGetLastError(); ncl = 0; }
             ncl = std::min(ncl, B);
-            if (ncl > 0) return true;
+            if (ncl > 0) return wins(ctx, B);
         }
         return false;
+    }
+    // B trajectories are ceil(B / ncl) rounds one after the other (7 clusters of 16 CTAs at a
+    // time), while k_fock_stage runs them side by side: as long as two CTAs each leave an SM to
+    // every CTA its time does not depend on B.  Per stage, in us, k_fock_stage against one round
+    // here, FP64: 8.6 and 3.0 at 9 sites, 11 and 3.5 at 16, 29 and 6.1 at 36, 99 and 11 at 64,
+    // 195 and 21 at 81, 890 and 56 at 119.  So the rounds that pay grow with n, by about one in
+    // ten sites; past one CTA per SM k_fock_stage slows down with B as well.  Measured time here
+    // over k_fock_stage's on either side: 12 sites, FP64, 12 trajectories 0.83, 18 1.13; 20
+    // sites 18 0.87, 24 1.09; 42 sites 36 0.91, 48 1.05; 64 sites 60 0.94, 66 1.04, 75 0.67,
+    // 150 0.87; 90 sites (Delta in global memory) 54 0.94, 60 1.05; 100 sites 100 0.90, 150
+    // 1.07; from 105 sites (FP32 from 80) below 1 up to 300 trajectories.
+    bool wins(const fpsg_ctx* ctx, int B) const
+    {
+        const int n = ctx->n, rounds = (B + ncl - 1) / ncl;
+        if (n >= (sizeof(R) == 4 ? 80 : 104)) return true;
+        if (!d_smem && n < 92) return rounds <= 7;
+        if (n >= 80) return B <= ctx->sm_count;
+        return rounds <= 2 + std::max(0, n - 4) / 10 || (n >= 60 && 2 * B > ctx->sm_count && B <= ctx->sm_count);
     }
 };
 

@@ -108,3 +108,21 @@ def test_fock_without_room_for_all_records():
     for k in ("niiu", "niid", "n2iiu", "n2iid", "nund"):
         assert np.array_equal(getattr(r, k), ref[k]), k
     eng.close()
+
+
+@pytest.mark.parametrize("n,B", [(4, 14), (4, 15), (4, 300), (30, 28), (30, 29), (64, 63), (64, 75)])
+def test_fock_ensembles(n, B):
+    """Ensembles on either side of the choice between the cluster kernel, round after round, and
+    the per-stage kernel: the same bits."""
+    T, U, V, ext, rng = small_system(n)
+    rho = hf_states(T, B, rng)
+    ref = orc.run(orc.System(T, U, V, ext, orc.COUL_DISTANCE, False), 1, 0.01, 1, 3, rho)
+    eng = E.Engine()
+    eng.set_system(T, U, V, ext, E.COUL_DISTANCE)
+    eng.set_initial_samples(rho)
+    r = eng.run(E.METHOD_HF, E.PREC_FP64, 0.01, 1, 3)
+    assert np.array_equal(eng.get_state(), ref["final"])
+    # means of B values of at most 1, summed in another order
+    for k in ("niiu", "niid", "n2iiu", "n2iid", "nund"):
+        assert np.max(np.abs(getattr(r, k) - ref[k])) < B * 2.0 ** -52, k
+    eng.close()
