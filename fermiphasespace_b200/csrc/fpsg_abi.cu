@@ -32,6 +32,7 @@ namespace {
 struct DevAlloc {
     void* p = nullptr;
     size_t bytes = 0;
+    bool batch = false;      // allocated for a system of a batch
 };
 
 template <typename R>
@@ -146,7 +147,7 @@ int dalloc(fpsg_ctx* ctx, void** p, size_t bytes)
         *p = nullptr;
         return fail(ctx, FPSG_ERR_OOM, std::string("cudaMalloc(") + std::to_string(bytes) + "): " + cudaGetErrorString(e));
     }
-    ctx->allocs.push_back({*p, bytes});
+    ctx->allocs.push_back({*p, bytes, ctx->pooled_state});
     ctx->mem_used += bytes;
     return FPSG_OK;
 }
@@ -2006,10 +2007,28 @@ void lend_pool(fpsg_ctx* from, fpsg_ctx* to)
     }
     from->pool.clear();
 }
-void release_sub(fpsg_ctx* c, fpsg_ctx* parent)
+// What the systems of a batch hold goes back to the parent's pool; under a memory cap it is
+// freed, and otherwise so are the blocks of earlier batches that this one had no use for, when
+// they are more than it used: the pool keeps at most twice the last batch's states and tables.
+void release_subs(std::vector<std::unique_ptr<fpsg_ctx>>& subs, fpsg_ctx* parent)
 {
-    c->pool = c->allocs;          // everything it holds
-    lend_pool(c, parent);
+    size_t used = 0, idle = 0;
+    std::vector<DevAlloc> other;
+    for (const DevAlloc& a : parent->pool)
+        if (a.batch) { idle += a.bytes; other.push_back(a); }
+    for (auto& c : subs) {
+        c->pool = c->allocs;          // everything it holds
+        used += c->mem_used;
+        lend_pool(c.get(), parent);
+    }
+    if (!parent->mem_cap && idle <= used) return;
+    std::vector<DevAlloc> keep, drop;
+    for (const DevAlloc& a : parent->pool) {
+        const bool mine = std::none_of(other.begin(), other.end(), [&](const DevAlloc& o) { return o.p == a.p; });
+        (a.batch && (parent->mem_cap || !mine) ? drop : keep).push_back(a);
+    }
+    parent->pool = keep;
+    for (const DevAlloc& a : drop) dfree(parent, a.p);
 }
 
 template <typename R>
@@ -2034,7 +2053,7 @@ int batch_impl(fpsg_ctx* ctx, const fpsg_system_desc* sd, int ns, int method, do
         if (rgraph) cudaGraphDestroy(rgraph);
         cudaStreamSynchronize(ctx->stream);     // pooled blocks may be written by the host next
         for (void* p : temps) trelease(ctx, p);
-        for (auto& c : subs) release_sub(c.get(), ctx);
+        release_subs(subs, ctx);
     };
     // systems and their samples, each in a context of its own
     for (int k = 0; k < ns; ++k) {
@@ -2519,6 +2538,10 @@ static int alloc_state(fpsg_ctx* ctx, int B)
     dfree(ctx, ctx->rho64); ctx->rho64 = nullptr; ctx->B = 0;
     const size_t bytes = sizeof(cplx<double>) * (size_t)B * 2 * ctx->ne;
     int rc = ctx->pooled_state ? talloc(ctx, (void**)&ctx->rho64, bytes) : dalloc(ctx, (void**)&ctx->rho64, bytes);
+    if (rc == FPSG_ERR_OOM && !ctx->pool.empty()) {       // scratch of earlier calls is in the way
+        trim_pool(ctx);
+        rc = dalloc(ctx, (void**)&ctx->rho64, bytes);
+    }
     if (rc) return rc;
     ctx->B = B;
     return FPSG_OK;
