@@ -883,6 +883,24 @@ struct FockLauncher {
     }
 };
 
+// k_stream_stage with the matrix in shared memory
+template <typename R>
+size_t stream_stage_smem(int n, int ne)
+{
+    return ((sizeof(cplx<R>) * ne + sizeof(R) * n + 15) & ~size_t(15)) + sizeof(double) * 32 * 4;
+}
+
+// With an offset pattern the pair stage, where a matrix has work for its 512 threads: it
+// takes 0.3 ms per stage against 0.7 (n = 256, FP32, 512 trajectories), and in shared
+// memory too k_stream_stage is the slower one (n = 143, FP64, 300 trajectories: 0.51
+// against 0.16 ms).
+template <typename R>
+bool takes_stream_pair(fpsg_ctx* ctx)
+{
+    return tables<R>(ctx).pat_ns != 0 &&
+           (stream_stage_smem<R>(ctx->n, ctx->ne) > ctx->smem_optin || ctx->n_pair >= 2 * SP_NT);
+}
+
 template <typename R>
 int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
 {
@@ -1044,7 +1062,7 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
             }
         }
         // stage the matrix in shared memory when it fits, else read it from global memory
-        size_t smem = ((sizeof(cplx<R>) * ne + sizeof(R) * n + 15) & ~size_t(15)) + sizeof(double) * 32 * 4;
+        size_t smem = stream_stage_smem<R>(n, ne);
         const bool gx = smem > ctx->smem_optin;
         if (gx) smem = ((sizeof(R) * n + 15) & ~size_t(15)) + sizeof(double) * 32 * 4;
         auto stage_fn = gx ? k_stream_stage<R, true> : k_stream_stage<R, false>;
@@ -1052,12 +1070,8 @@ int run_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
         int per_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stage_fn, 256, smem));
         const int grid = std::max(1, std::min(2 * B, std::max(1, per_sm) * ctx->sm_count));
-        // With an offset pattern the pair stage, where a matrix has work for its 512 threads: it
-        // takes 0.3 ms per stage against 0.7 (n = 256, FP32, 512 trajectories), and in shared
-        // memory too k_stream_stage is the slower one (n = 143, FP64, 300 trajectories: 0.51
-        // against 0.16 ms).
         const DevTables<R>& tb = tables<R>(ctx);
-        const bool sp = !fock && tb.pat_ns != 0 && (gx || ctx->n_pair >= 2 * SP_NT);
+        const bool sp = !fock && takes_stream_pair<R>(ctx);
         auto sp_fn = tb.pat_ns == 3 ? k_stream_pair<R, 3> : k_stream_pair<R, 2>;
         const size_t sp_smem = stream_pair_smem(n, sizeof(R));
         int sp_grid = 1;
@@ -2236,6 +2250,8 @@ int batch_impl(fpsg_ctx* ctx, const fpsg_system_desc* sd, int ns, int method, do
                 a.do_e1 = (hf ? (c->coul != FPSG_COULOMB_NULL) : 1) && rec_e;
                 a.do_e2 = (hf ? 0 : 1) && rec_e;
                 a.diagbuf = b.diagbuf; a.ebuf = b.ebuf; a.whole = nullptr; a.err = d_err;
+                // a system run by itself gives the same bits
+                a.diag_apart = takes_stream_pair<R>(c) ? 1 : 0;
             }
         StreamArgs<R>* args = nullptr;
         if ((rc = tmp((void**)&args, sizeof(StreamArgs<R>) * ha.size()))) { cleanup(); return rc; }

@@ -136,25 +136,33 @@ __device__ __forceinline__ R delta_diag(const DevSys<R>& s, int j, const cplx<R>
     return d;
 }
 
-// k = -i (X Delta - Delta X) at (i, j), X packed, Delta diagonal in Dd.
-template <typename R>
+// k = -i (X Delta - Delta X) at (i, j), X packed, Delta diagonal in Dd.  APART: the diagonal
+// terms of both sums as one, X_ij (Delta_jj - Delta_ii), the way k_stream_pair has it in FP32
+// (in the sums they take the weight 0: a test per entry costs 13 % of k_batch_stage).
+template <typename R, bool APART = false>
 __device__ __forceinline__ cplx<R> commutator_elem(const DevSys<R>& s, const cplx<R>* __restrict__ X,
                                                    const R* __restrict__ Dd, int i, int j)
 {
     R are = R(0), aim = R(0), bre = R(0), bim = R(0);
     for (int q = s.hp[j]; q < s.hp[j + 1]; ++q) {
         const int k = s.hk[q];
-        const R d = (k == j) ? Dd[j] : s.hv[q];
+        const R d = (k == j) ? (APART ? R(0) : Dd[j]) : s.hv[q];
         const cplx<R> x = getH<R>(X, i, k);
         are = fmaR<R>(x.re, d, are);
         aim = fmaR<R>(x.im, d, aim);
     }
     for (int q = s.hp[i]; q < s.hp[i + 1]; ++q) {
         const int k = s.hk[q];
-        const R d = (k == i) ? Dd[i] : s.hv[q];
+        const R d = (k == i) ? (APART ? R(0) : Dd[i]) : s.hv[q];
         const cplx<R> x = getH<R>(X, k, j);
         bre = fmaR<R>(x.re, d, bre);
         bim = fmaR<R>(x.im, d, bim);
+    }
+    if constexpr (APART) {
+        const cplx<R> x = X[cs(j) + i];
+        const R d = Dd[j] - Dd[i];
+        are = fmaR<R>(x.re, d, are);
+        aim = fmaR<R>(x.im, d, aim);
     }
     cplx<R> r;
     r.re = subR<R>(aim, bim);

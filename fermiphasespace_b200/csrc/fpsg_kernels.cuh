@@ -90,13 +90,14 @@ struct StreamArgs {
     double* ebuf;      // [B][2][4]  per-trajectory energy partials
     double2* whole;    // [2][ne] running sums of rho (or null)
     unsigned* err;
+    int diag_apart = 0;    // FP32: the diagonal terms once, as X_ij (Delta_jj - Delta_ii)
 };
 
 // One RK stage of spin matrix m (the body of the stream kernels).  GX = false
 // stages the matrix in shared memory; GX = true reads it from global memory
 // (through L1/L2) for n whose packed matrix exceeds shared memory.  Both do the
 // same arithmetic in the same order.  Every thread of the CTA takes part.
-template <typename R, bool GX>
+template <typename R, bool GX, bool APART = false>
 __device__ __forceinline__ void stream_matrix(const StreamArgs<R>& a, int m, unsigned char* smem)
 {
     const int n = a.sys.n, ne = a.sys.ne;
@@ -142,7 +143,7 @@ __device__ __forceinline__ void stream_matrix(const StreamArgs<R>& a, int m, uns
     for (int p = threadIdx.x; p < ne; p += blockDim.x) {
         const uint32_t ij = a.sys.pij[p];
         const int i = ij & 0xffff, j = ij >> 16;
-        const cplx<R> k = commutator_elem<R>(a.sys, X, Dd, i, j);
+        const cplx<R> k = commutator_elem<R, APART>(a.sys, X, Dd, i, j);
         const size_t g = (size_t)m * ne + p;
         const cplx<R> z = {R(0), R(0)};
         cplx<R> rho = (a.stage == 0) ? X[p] : a.rho[g];
@@ -176,6 +177,11 @@ __global__ void __launch_bounds__(512) k_batch_stage(const StreamArgs<R>* __rest
     extern __shared__ __align__(16) unsigned char smem[];
     for (int q = blockIdx.x; q < n_items; q += gridDim.x) {
         const int2 it = items[q];
+        if constexpr (std::is_same<R, float>::value)
+            if (args[it.x].diag_apart) {
+                stream_matrix<R, GX, true>(args[it.x], it.y, smem);
+                continue;
+            }
         stream_matrix<R, GX>(args[it.x], it.y, smem);
     }
 }
