@@ -1487,16 +1487,27 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
         const size_t traj = sizeof(cplx<R>) * 2 * (size_t)ne;
         const size_t per_keep = traj * 4 * (size_t)C * (size_t)nseg;          // every segment kept
         const size_t per_tmp = traj * (size_t)(10 + nck + 4 * C);              // the chunk's scratch
-        size_t fre = 0, tot = 0, pooled = 0, largest = 0;
-        for (const auto& a : ctx->pool) {
-            pooled += a.bytes;
-            largest = std::max(largest, a.bytes);
+        size_t fre = 0, tot = 0, pooled = 0;
+        int bi = -1;                                                           // the largest pooled block
+        for (int i = 0; i < (int)ctx->pool.size(); ++i) {
+            pooled += ctx->pool[i].bytes;
+            if (bi < 0 || ctx->pool[i].bytes > ctx->pool[bi].bytes) bi = i;
         }
-        // A pooled buffer that holds every stage input of the whole ensemble (a previous call of
-        // this shape left it) needs no look at the free memory, a driver call that has been seen
-        // to take tens of milliseconds on a busy host.
-        const bool fits = largest >= (size_t)Ball * per_keep;
-        if (!fits && cudaMemGetInfo(&fre, &tot) != cudaSuccess) { cudaGetLastError(); fre = 0; }
+        // When one pooled block holds every stage input of the whole ensemble and the others as
+        // much as the scratch beside it takes (a previous call of this shape left them), the call
+        // needs no memory that it does not have: one chunk, without a look at the free memory, a
+        // driver call that has been seen to take tens of milliseconds on a busy host.  The block
+        // is set aside, so that no other request takes or frees it.
+        const bool fits = bi >= 0 && !ctx->mem_cap && ctx->grad_keep < 0 &&
+                          ctx->pool[bi].bytes >= (size_t)Ball * per_keep &&
+                          pooled - ctx->pool[bi].bytes >= (size_t)Ball * per_tmp;
+        if (fits) {
+            keep = (cplx<R>*)ctx->pool[bi].p;
+            ctx->pool.erase(ctx->pool.begin() + bi);
+        } else if (cudaMemGetInfo(&fre, &tot) != cudaSuccess) {
+            cudaGetLastError();
+            fre = 0;
+        }
         size_t avail = fre + pooled;       // pooled scratch is reused or released
         if (ctx->mem_cap) {
             const size_t held = ctx->mem_used > pooled ? ctx->mem_used - pooled : 0;
@@ -1518,7 +1529,7 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
         }
     }
     const size_t count = (size_t)B * 2 * ne;
-    int n_keep = 0;                                            // segments kept from the sweep
+    int n_keep = keep ? (int)nseg : 0;                         // segments kept from the sweep
     cplx<R> *st, *A, *Bc, *X0, *X1, *ck, *seg, *lam, *xb;
     R* dbar;
     double *pacc, *diagbuf, *ebuf, *part, *sums, *pout;
@@ -1634,7 +1645,7 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
         // pooled block when it holds at least as many segments as a new buffer could,
         // since memory written before is much faster to fill than a fresh allocation
         // of tens of GB.
-        if (Nsteps > 0 && ctx->grad_keep != 0) {
+        if (Nsteps > 0 && ctx->grad_keep != 0 && !keep) {
             const size_t segbytes = sizeof(cplx<R>) * count * 4 * (size_t)C;
             const long want = ctx->grad_keep > 0 ? std::min<long>(nseg, (long)((size_t)ctx->grad_keep / segbytes)) : nseg;
             int bi = -1;

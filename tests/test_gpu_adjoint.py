@@ -300,3 +300,29 @@ def test_segment_kernel_configurations(engine_lib, dims):
             assert abs(a["loss"] - b["loss"]) < tol
             for k in ("dU", "dt", "dpulse"):
                 assert np.max(np.abs(a[k] - b[k])) < tol * scale, (k, prec)
+
+
+def test_plan_does_not_depend_on_what_the_pool_holds(engine_lib):
+    """A call after one of another checkpoint interval, under a memory cap: the block of stage
+    inputs that the first call left is large enough for the second one's, but not with the
+    scratch beside it.  The plan is that of a new context."""
+    E = engine_lib
+    B, n = 600, 9
+    T = configs.hopping(configs.distances(configs.grid_positions(3, 3)), [(1.0, -1.0)])
+    occ = (np.arange(n) % 2).astype(float)
+    traj = 32 * n * (n + 1) // 2                 # bytes of a trajectory
+    out = []
+    for first in (True, False):
+        eng = E.Engine()
+        eng.set_memory_cap(320 * B * traj)
+        eng.set_system(T, 3.0 * np.eye(n), None, None, coulomb=E.COUL_ONSITE)
+        eng.sample(B, 3, occ, 1.0 - occ)
+        if first:
+            a = eng.grad(E.PREC_FP64, 0.01, 1, 41, checkpoint_every=1)     # 160 + 55 of the 320
+            assert a["chunks"] == 1 and a["kept_segments"] == a["segments"] == 40
+        out.append(eng.grad(E.PREC_FP64, 0.01, 1, 41, checkpoint_every=20))  # 160 + 93
+        eng.close()
+    for k in ("chunk_traj", "chunks", "segments", "kept_segments"):
+        assert out[0][k] == out[1][k], k
+    for k in ("dU", "dt"):
+        assert out[0][k] == out[1][k], k
