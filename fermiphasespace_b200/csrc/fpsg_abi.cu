@@ -80,6 +80,7 @@ struct fpsg_ctx {
     std::vector<DevAlloc> pool;            // per-call scratch kept for the next call (counted in mem_used)
     bool pooled_state = false;             // the state comes from the pool (systems of a batch)
     int64_t grad_keep = -1;                // fpsg_set_grad_memory: -1 automatic
+    int clusters4 = -1;                    // 4-CTA clusters, a CTA per SM, that run at a time (-1: not asked yet)
     fpsg_grad_info grad_info = {0, 0, 0, 0};   // the last fpsg_grad call's plan
 
     // system
@@ -617,10 +618,36 @@ ResPlan plan_resident(fpsg_ctx* ctx, int B, bool comp = false)
     return plan.idx < 0 ? plan_resident_of<R>(ctx, B, comp, false) : plan;
 }
 
-// One wave of 4-CTA clusters (four SMs per trajectory) ends before one of 2-CTA clusters
-// does (10x10 grid, FP64, 1 trajectory x 400 steps: 10.3 against 13.0 ms), but only a quarter
-// of the SM count of them run at a time.
-bool few_trajectories(const fpsg_ctx* ctx, int B) { return B <= ctx->sm_count / 5; }
+// One wave of 4-CTA clusters (four SMs per trajectory) ends before one of 2-CTA clusters does, but
+// the device runs only some 33 of them at a time, and the trajectory after them would wait for a
+// second wave.  20 steps, 33 and 34 trajectories, four SMs each against two: 10x10 grid, FP64, 0.478
+// and 0.932 against 0.584 ms; fcc 72, FP64, 0.832 and 1.65 against 1.07; 12x12 grid, FP32, 0.785
+// and 1.52 against 0.995 (k_pair_packed with 11 slots a thread; 11x11 with 8: 0.736 against 0.523).
+bool few_trajectories(fpsg_ctx* ctx, int B)
+{
+    if (B > ctx->sm_count / 4) return false;
+    if (ctx->clusters4 < 0) {
+        ctx->clusters4 = ctx->sm_count / 5;
+        for (const QuadCfg<double>& c : quad_hp_cfgs<double>()) {
+            if (c.nh != 2) continue;
+            const size_t smem = ctx->smem_optin - 4096;                 // one CTA per SM
+            cudaLaunchConfig_t lc = {};
+            lc.gridDim = dim3(ctx->sm_count); lc.blockDim = dim3(c.nt); lc.dynamicSmemBytes = smem; lc.stream = ctx->stream;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = 4; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+            lc.attrs = at; lc.numAttrs = 1;
+            int n = 0;
+            if (allow_smem(ctx, (const void*)c.fn[0], smem) == cudaSuccess &&
+                cudaOccupancyMaxActiveClusters(&n, (void*)c.fn[0], &lc) == cudaSuccess && n > 0)
+                ctx->clusters4 = n;
+            else
+                cudaGetLastError();
+            break;
+        }
+    }
+    return B <= ctx->clusters4;
+}
 
 // The 4-CTA-cluster kernel for matrices too large for k_resident: the smallest
 // elements-per-thread whose half-matrix slots cover both halves and whose shared
@@ -647,7 +674,7 @@ ResPlan plan_quad(fpsg_ctx* ctx, bool comp, int B)
         for (int c = 0; c < (int)hf.size(); ++c) {
             const int nh = hf[c].nh;
             if (nh == 2 && !(std::is_same<R, double>::value || Wc <= 5)) continue;
-            // few FP64 trajectories: four SMs for each (see choose_resident)
+            // few FP64 trajectories: four SMs for each
             if (nh == 1 && std::is_same<R, double>::value && few_trajectories(ctx, B)) continue;
             const int cap = hf[c].nt * hf[c].ept;
             if (cap < (nh == 2 ? need : ne)) continue;
@@ -702,8 +729,8 @@ ResPlan choose_resident(fpsg_ctx* ctx, int B)
         const ResPlan pk = plan_packed<R>(ctx, comp_ok);
         if (pk.idx >= 0) {
             plan = pk;
-            if (std::is_same<R, double>::value && few_trajectories(ctx, B)) {
-                const ResPlan two = plan_quad<R>(ctx, false, B);
+            if ((std::is_same<R, double>::value || packed_cfgs<R>()[pk.idx].ept > 8) && few_trajectories(ctx, B)) {
+                const ResPlan two = plan_quad<R>(ctx, comp_ok, B);
                 if (two.idx >= 0 && two.hp && two.nh == 2) plan = two;
             }
             return plan;
@@ -2085,7 +2112,7 @@ int batch_impl(fpsg_ctx* ctx, const fpsg_system_desc* sd, int ns, int method, do
         subs.emplace_back(new fpsg_ctx());
         fpsg_ctx* c = subs.back().get();
         c->device = ctx->device; c->sm_count = ctx->sm_count; c->smem_optin = ctx->smem_optin;
-        c->stream = ctx->stream; c->ev0 = ctx->ev0; c->ev1 = ctx->ev1; c->flags = ctx->flags;
+        c->stream = ctx->stream; c->ev0 = ctx->ev0; c->ev1 = ctx->ev1; c->flags = ctx->flags; c->clusters4 = ctx->clusters4;
         lend_pool(ctx, c);
         c->pooled_state = true;
         // what the parent holds beside its pool counts against the cap
