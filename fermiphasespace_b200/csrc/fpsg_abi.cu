@@ -610,12 +610,32 @@ ResPlan plan_resident_of(fpsg_ctx* ctx, int B, bool comp, bool pair)
 // The pair kernels wherever Delta has an offset pattern and a configuration fits: they
 // need fewer shared-memory wavefronts per element than the column kernels at every P
 // such a Delta can have (fpsg_pair.cuh), also where half of the slots is masked
-// (three offsets and three neighbours per site, as the honeycomb lattice has).
+// (three offsets and three neighbours per site, as the honeycomb lattice has).  The kernel
+// depends on the system alone, so that fpsg_grad's chunks of an ensemble give its bits.
 template <typename R>
 ResPlan plan_resident(fpsg_ctx* ctx, int B, bool comp = false)
 {
     const ResPlan plan = plan_resident_of<R>(ctx, B, comp, true);
     return plan.idx < 0 ? plan_resident_of<R>(ctx, B, comp, false) : plan;
+}
+
+// Where the column kernel has a thread for each element, and so few of them per SM that nothing
+// but the length of a thread's chain counts, it is faster than the pair kernel: its thread forms
+// one element, the pair kernel's two.  40 steps, columns against pairs, elements per SM in
+// brackets: FP64, 6 sites, 148 trajectories (42) 68 against 98 us, 300 (168) 97 against 111, 5
+// sites, 1000 (240) 127 against 116; FP32, 6 sites, 148 (42) 62 against 70, 5 sites, 1000 (240)
+// 77 against 98, 6 sites, 1000 (378) 103 against 104.
+template <typename R>
+bool columns_win(fpsg_ctx* ctx, int B, bool comp, ResPlan& plan)
+{
+    if (!plan.pair || ctx->n > 10 || tables<R>(ctx).ud) return false;
+    const ResPlan col = plan_resident_of<R>(ctx, B, comp, false);
+    if (col.idx < 0) return false;
+    const ResCfg<R>& cf = res_cfgs<R>()[col.idx];
+    const int groups = (B + col.G - 1) / col.G, per_sm = (groups + ctx->sm_count - 1) / ctx->sm_count;
+    if (cf.ept != 1 || cf.split || per_sm * 2 * col.G * ctx->ne > (sizeof(R) == 8 ? 180 : 256)) return false;
+    plan = col;
+    return true;
 }
 
 // One wave of 4-CTA clusters (four SMs per trajectory) ends before one of 2-CTA clusters does, but
@@ -724,6 +744,7 @@ ResPlan choose_resident(fpsg_ctx* ctx, int B)
 {
     const bool comp_ok = !std::is_same<R, double>::value && !(ctx->flags & FPSG_FLAG_FP32_PLAIN_STATE);
     ResPlan plan = plan_resident<R>(ctx, B, comp_ok);
+    if (columns_win<R>(ctx, B, comp_ok, plan)) return plan;
     // k_pair_packed where k_pair does not fit, before anything without the compensated update
     if (plan.idx < 0 || !plan.pair) {
         const ResPlan pk = plan_packed<R>(ctx, comp_ok);
