@@ -694,8 +694,10 @@ ResPlan plan_quad(fpsg_ctx* ctx, bool comp, int B)
         for (int c = 0; c < (int)hf.size(); ++c) {
             const int nh = hf[c].nh;
             if (nh == 2 && !(std::is_same<R, double>::value || Wc <= 5)) continue;
-            // few FP64 trajectories: four SMs for each
-            if (nh == 1 && std::is_same<R, double>::value && few_trajectories(ctx, B)) continue;
+            // few FP64 trajectories: four SMs for each, where a CTA's share is worth the exchange (20
+            // steps, 1 to 33 trajectories, one CTA per spin against two: moire 16 0.39 against
+            // 0.66 ms, fcc 32 0.44 against 0.43, fcc 48 0.56 against 0.51)
+            if (nh == 1 && std::is_same<R, double>::value && ne > 500 && few_trajectories(ctx, B)) continue;
             const int cap = hf[c].nt * hf[c].ept;
             if (cap < (nh == 2 ? need : ne)) continue;
             const size_t sm = quad_hp_layout<R>(n, Wc, cap, e8).total;
