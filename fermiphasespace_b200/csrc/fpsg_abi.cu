@@ -1575,7 +1575,9 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
             B = (int)((Ball + nchunk - 1) / nchunk);
             B = ((B + q - 1) / q) * q;
             if (B >= Ball) B = Ball;
-            else plan = plan_resident<R>(ctx, B);
+            // (FP32 with dense Coulomb rows keeps the whole ensemble's plan: how a CTA splits those
+            // sums, and so a trajectory's bits, goes by the number of its trajectories)
+            else if (std::is_same<R, double>::value || !tables<R>(ctx).ud) plan = plan_resident<R>(ctx, B);
         }
     }
     const size_t count = (size_t)B * 2 * ne;

@@ -326,3 +326,32 @@ def test_plan_does_not_depend_on_what_the_pool_holds(engine_lib):
         assert out[0][k] == out[1][k], k
     for k in ("dU", "dt"):
         assert out[0][k] == out[1][k], k
+
+
+@pytest.mark.parametrize("dims", [(5, 5), (6, 6)])
+def test_fp32_distance_coulomb_chunks(engine_lib, oracle_lib, dims):
+    """FP32 with dense Coulomb rows, whose sums are split among the threads that a CTA has to spare:
+    the gradients of chunks are still those of the whole ensemble, to the bit."""
+    import torch
+    E, O = engine_lib, oracle_lib
+    D = configs.distances(configs.grid_positions(*dims))
+    n = D.shape[0]
+    T = configs.hopping(D, [(1.0, -1.0)])
+    U = 2.0 / (1.0 + D)
+    V = U - np.diag(np.diag(U))
+    occ = (np.arange(n) % 2).astype(float)
+    sm = torch.cuda.get_device_properties(0).multi_processor_count
+    B, C, S, Tp = 3 * sm, 5, 1, 11
+    nseg = (Tp - 1 + C - 1) // C
+    per_traj = 8 * 2 * (n * (n + 1) // 2) * 4 * C * nseg     # every segment of one trajectory
+    eng = E.Engine()
+    eng.set_system(T, U, V, None, coulomb=E.COUL_DISTANCE)
+    res = []
+    for budget in (-1, per_traj * sm):
+        eng.sample(B, 17, occ, 1.0 - occ)
+        eng.set_grad_memory(budget)
+        res.append(eng.grad(E.PREC_FP32, 0.02, S, Tp, checkpoint_every=C))
+    assert (res[0]["chunks"], res[1]["chunks"]) == (1, 3)
+    for k in ("dU", "dt"):
+        assert res[0][k] == res[1][k], k
+    eng.close()
