@@ -1316,16 +1316,14 @@ int dense_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
     };
     auto cleanup = [&]() { for (void* p : temps) trelease(ctx, p); };
     const size_t mat = (size_t)M * 2 * NP * NP;
-    float *R = nullptr, *Xa = nullptr, *Xb = nullptr, *Xc = nullptr, *Tf = nullptr, *Ud = nullptr, *Vd = nullptr,
-          *dvec = nullptr;
+    float *R = nullptr, *Xa = nullptr, *Xb = nullptr, *Xc = nullptr, *Tf = nullptr, *Ud = nullptr, *Vd = nullptr;
     void* Tc = nullptr;
     const bool tf32 = q.precision == FPSG_PREC_SPLIT_TF32X3;
     unsigned* d_err = nullptr;
     if ((rc = tmp((void**)&R, sizeof(float) * mat)) || (rc = tmp((void**)&Xa, sizeof(float) * mat)) ||
         (rc = tmp((void**)&Xb, sizeof(float) * mat)) || (rc = tmp((void**)&Xc, sizeof(float) * mat)) ||
         (rc = tmp((void**)&Tf, sizeof(float) * NP * NP)) ||
-        (rc = tmp(&Tc, TC_BYTES)) || (rc = tmp((void**)&dvec, sizeof(float) * (size_t)M * NP)) ||
-        (rc = tmp((void**)&d_err, sizeof(unsigned)))) {
+        (rc = tmp(&Tc, TC_BYTES)) || (rc = tmp((void**)&d_err, sizeof(unsigned)))) {
         cleanup();
         return rc;
     }
@@ -1370,15 +1368,23 @@ int dense_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
     const int chunk = 64, nch = (B + chunk - 1) / chunk;
     const int do_e1 = hf ? (ctx->coul != FPSG_COULOMB_NULL) : 1;
     const int rec_e = (q.obs & FPSG_OBS_ENERGIES) ? 1 : 0;
+    float* Et = nullptr;
+    bool planes = q.record && !(q.obs & FPSG_OBS_WHOLE);
     if (q.record) {
         if ((rc = tmp((void**)&sums, sizeof(double) * (size_t)q.Tp * W)) ||
             (rc = tmp((void**)&diagbuf, sizeof(double) * (size_t)B * 2 * n)) ||
             (rc = tmp((void**)&ebuf, sizeof(double) * (size_t)B * 2 * 4)) ||
-            (rc = tmp((void**)&part, sizeof(double) * (size_t)nch * W)) ||
-            ((q.obs & FPSG_OBS_WHOLE) && (rc = tmp((void**)&packed, sizeof(cplx<float>) * (size_t)M * ne)))) {
+            (rc = tmp((void**)&part, sizeof(double) * (size_t)nch * W))) {
             cleanup();
             return rc;
         }
+        // records straight from the planes need the static potential in plane order; without room
+        // for it, as for whole matrices, they go through a packed copy
+        if (planes && !ctx->ext_null && tmp((void**)&Et, sizeof(float) * NP * NP)) {
+            ctx->err.clear();
+            planes = false;
+        }
+        if (!planes && (rc = tmp((void**)&packed, sizeof(cplx<float>) * (size_t)M * ne))) { cleanup(); return rc; }
         CK(cudaMemsetAsync(ebuf, 0, sizeof(double) * (size_t)B * 2 * 4, ctx->stream));
         if (q.obs & FPSG_OBS_WHOLE) {
             if ((rc = tmp((void**)&whole, sizeof(double2) * (size_t)q.Tp * 2 * ne))) { cleanup(); return rc; }
@@ -1393,7 +1399,10 @@ int dense_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
     const int grid = std::max(1, std::min(M, ctx->sm_count));
 
     DenseArgs da;
-    da.n = n; da.M = M; da.Tc = Tc; da.sys = sys; da.err = d_err; da.Ud = Ud; da.Vd = Vd; da.dvec = dvec;
+    da.n = n; da.M = M; da.Tc = Tc; da.sys = sys; da.err = d_err; da.Ud = Ud; da.Vd = Vd;
+    // 4 steps, n = 16, without and with: 48 matrices 0.902 and 0.914 ms, 64 0.957 and 0.935, 148
+    // 1.29 and 1.24
+    da.prefetch = 5 * M > 2 * ctx->sm_count;
     // test hook: the call's first launch waits on a barrier nothing arrives at
     da.probe_polls = (ctx->flags & FPSG_FLAG_TEST_EXPIRE_WAIT) ? 4096u : 0u;
     double tc = q.record ? 0.0 : q.t_start;
@@ -1407,36 +1416,34 @@ int dense_impl(fpsg_ctx* ctx, const RunReq& q, RunOut& out)
             case 2: da.X = Xb; da.P0 = Xa;      da.P1 = nullptr; da.a0 = 2.f;  da.a1 = 0.f;   da.ax = -1.f;   da.hk = hf32;       da.out = Xc; break;
             default: da.X = Xc; da.P0 = R;      da.P1 = Xb;      da.a0 = -0.125f; da.a1 = 0.75f; da.ax = 0.375f; da.hk = hf32 / 8.f; da.out = R; break;
             }
+            // the diagonals' own launch for dense Coulomb rows and more than five matrices per CTA
+            // (see k_dense_diag); they wait in a buffer that the stage does not read: its output, or
+            // X2 in the last one
+            da.dvec = !Ud || M <= 5 * ctx->sm_count ? nullptr : g == 3 ? Xa : da.out;
             CK(launch_stage(da, grid, tf32, ctx->stream));
             da.probe_polls = 0;
-            out.launches += 2;
+            out.launches += da.dvec ? 2 : 1;
         }
         tc += h;
         return FPSG_OK;
     };
-    // tM and the static potential in plane order, for the records
+    // tM (in place of the matrix that prep_T has read) and the static potential in plane order
     DenseRecordArgs dr = {};
-    if (q.record && !whole) {
+    if (planes) {
         std::vector<float> th((size_t)NP * NP, 0.f), eh((size_t)NP * NP, 0.f);
         for (int j = 0; j < n; ++j)
             for (int i = 0; i < n; ++i) {
                 th[plane_off(i, j)] = (float)ctx->tM[(size_t)j * n + i];
                 if (!ctx->ext_null) eh[plane_off(i, j)] = (float)ctx->ext[(size_t)j * n + i];
             }
-        float *tt = nullptr, *et = nullptr;
-        if ((rc = tmp((void**)&tt, sizeof(float) * th.size())) ||
-            (!ctx->ext_null && (rc = tmp((void**)&et, sizeof(float) * eh.size())))) {
-            cleanup();
-            return rc;
-        }
-        CK(cudaMemcpyAsync(tt, th.data(), sizeof(float) * th.size(), cudaMemcpyHostToDevice, ctx->stream));
-        if (et) CK(cudaMemcpyAsync(et, eh.data(), sizeof(float) * eh.size(), cudaMemcpyHostToDevice, ctx->stream));
+        CK(cudaMemcpyAsync(Tf, th.data(), sizeof(float) * th.size(), cudaMemcpyHostToDevice, ctx->stream));
+        if (Et) CK(cudaMemcpyAsync(Et, eh.data(), sizeof(float) * eh.size(), cudaMemcpyHostToDevice, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
-        dr.n = n; dr.B = B; dr.X = R; dr.Tt = tt; dr.Et = et; dr.Ud = Ud; dr.Vd = Vd; dr.sys = sys;
+        dr.n = n; dr.B = B; dr.X = R; dr.Tt = Tf; dr.Et = Et; dr.Ud = Ud; dr.Vd = Vd; dr.sys = sys;
         dr.do_en = rec_e; dr.do_e1 = sa.do_e1; dr.do_e2 = sa.do_e2; dr.diagbuf = diagbuf; dr.ebuf = ebuf; dr.err = d_err;
     }
     auto record = [&](int t) -> int {
-        if (!whole) {
+        if (planes) {
             CK(launch_record(dr, ctx->stream));
             k_reduce_part<<<dim3(nch, 1, (W + 255) / 256), 256, 0, ctx->stream>>>(diagbuf, ebuf, B, n, chunk, part);
             k_reduce_fin<<<std::max(1, (W + 255) / 256), 256, 0, ctx->stream>>>(part, nch, W, sums + (size_t)t * W);

@@ -68,6 +68,7 @@ __host__ __device__ __forceinline__ int canon(int r, int k)
 struct Shared {
     // after the stage buffers
     float d[2][NP];          // Delta_jj of the matrix (double-buffered by matrix)
+    float nd[2][NP];         // n_jj + shift of the other and of the same spin (DenseArgs::dvec null)
     uint64_t fullX[STAGES];  // producers' conversions done (an arrival per warp)
     uint64_t fullT[STAGES];  // T bulk copies landed (1 arrival + bytes)
     uint64_t empty[STAGES];  // MMAs reading the stage are done
@@ -158,6 +159,32 @@ __device__ __forceinline__ void epi_prefetch(const DenseArgs& a, int m, int p, i
     if (a.P1) tc::prefetch_l2(a.P1 + oq, bytes);
 }
 
+// Delta_jj = ((tM_jj + sum U (n_other + s)) + sum V (n_same + s)) + ext_jj + pulse proj_j from the
+// densities n + s of both spins, by the operations of k_dense_diag
+__device__ __forceinline__ float diag_site(const DenseArgs& a, int j, const float* other, const float* same)
+{
+    if (j >= a.n) return 0.f;
+    const DevSys<float>& sy = a.sys;
+    float u = 0.f, v = 0.f;
+    if (a.Ud) {
+#pragma unroll 8
+        for (int k = 0; k < a.n; ++k) {
+            u = fmaf(__ldg(a.Ud + (size_t)k * NP + j), other[k], u);
+            v = fmaf(__ldg(a.Vd + (size_t)k * NP + j), same[k], v);
+        }
+    } else if (sy.coul != 0) {
+        for (int x = sy.up[j]; x < sy.up[j + 1]; ++x) u = fmaf(sy.uv[x], other[sy.uk[x]], u);
+        if (sy.coul == 2)
+            for (int x = sy.vp[j]; x < sy.vp[j + 1]; ++x) v = fmaf(sy.vv[x], same[sy.vk[x]], v);
+    }
+    float d = sy.tdiag[j];
+    if (sy.coul != 0) d += u;
+    if (sy.coul == 2) d += v;
+    if (sy.has_ext) d += sy.ediag[j];
+    if (sy.n_bins > 0) d += a.pulse * sy.proj[j];
+    return d;
+}
+
 template <bool TF32>
 __global__ void __launch_bounds__(NTHREADS, 1) k_dense_stage(DenseArgs a)
 {
@@ -218,7 +245,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_dense_stage(DenseArgs a)
                 for (int kc = 0; kc < NCHE; ++kc, ++it) {
                     const int s = it % STAGES;
                     // the chunk two on into L2: 8 row blocks of KCE columns, contiguous each
-                    if (pw == 0 && lane < NP / 32 && kc + 2 < NCHE)
+                    if (pw == 0 && lane < NP / 32 && kc + 2 < NCHE && a.prefetch)
                         tc::prefetch_l2(Xp + plane_off(lane * 32, (kc + 2) * KCE), 32 * KCE * sizeof(float));
                     // the loads go out before the stage is free
                     // lane (r8, kq): one 16-byte core row of row r, K-core kq
@@ -230,10 +257,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_dense_stage(DenseArgs a)
                         v[q][0] = __ldg(reinterpret_cast<const float4*>(Xp + plane_off(r, k)));
                         if constexpr (!TF32) v[q][TF32 ? 0 : 1] = __ldg(reinterpret_cast<const float4*>(Xp + plane_off(r, k + 4)));
                     }
-                    // one lane polls; the outcome is the warp's
-                    uint32_t got = 1;
-                    if (lane == 0) got = wait_bar(&sh->empty[s], ((it / STAGES) & 1) ^ 1, sh, a.err) ? 1u : 0u;
-                    if (!__shfl_sync(0xffffffffu, got, 0)) { ok = false; break; }
+                    if (!wait_bar(&sh->empty[s], ((it / STAGES) & 1) ^ 1, sh, a.err)) { ok = false; break; }
                     unsigned char* st = stages + (size_t)s * STAGE_BYTES;
                     if (pt == 0) {
                         const char* tcb = reinterpret_cast<const char*>(a.Tc);
@@ -334,7 +358,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_dense_stage(DenseArgs a)
         bool ok = true;
         for (int m = blockIdx.x; m < a.M && ok; m += gridDim.x, ++mi) {
             const float* Xm = a.X + (size_t)m * mstride;
-            for (int j = et; j < NP; j += N_EPI_WARPS * 32) sh->d[mi & 1][j] = __ldg(a.dvec + (size_t)m * NP + j);
+            if (a.dvec) {
+                for (int j = et; j < NP; j += N_EPI_WARPS * 32) sh->d[mi & 1][j] = __ldcg(a.dvec + (size_t)m * mstride + j);
+            } else {
+                const float* Xo = a.X + (size_t)(m ^ 1) * mstride;
+                for (int j = et; j < NP; j += N_EPI_WARPS * 32) {
+                    sh->nd[0][j] = j < a.n ? Xo[plane_off(j, j)] + a.sys.shift : 0.f;
+                    sh->nd[1][j] = j < a.n ? Xm[plane_off(j, j)] + a.sys.shift : 0.f;
+                }
+                tc::named_sync(1, N_EPI_WARPS * 32);
+                for (int j = et; j < NP; j += N_EPI_WARPS * 32) sh->d[mi & 1][j] = diag_site(a, j, sh->nd[0], sh->nd[1]);
+            }
             tc::named_sync(1, N_EPI_WARPS * 32);
             const float* dd = sh->d[mi & 1];
             for (int p = 0; p < 2 && ok; ++p) {
@@ -359,7 +393,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_dense_stage(DenseArgs a)
 #pragma unroll 1
                     for (int jb = 0; jb < EPI_COLS / EPI_BLK; ++jb) {
                         const int j0 = hh * EPI_COLS + jb * EPI_BLK;
-                        if (lane == 0) epi_prefetch(a, m, p, mt, q4, hh, jb + EPI_AHEAD);
+                        if (lane == 0 && a.prefetch) epi_prefetch(a, m, p, mt, q4, hh, jb + EPI_AHEAD);
                         // global loads first: their latency overlaps the tensor-memory read
                         const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
                         float4 vp[EPI_BLK / 4], vq[EPI_BLK / 4], v0[EPI_BLK / 4], v1[EPI_BLK / 4];
@@ -407,11 +441,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_dense_stage(DenseArgs a)
     }
 }
 
-// Delta_jj = ((tM_jj + sum U (n_other + s)) + sum V (n_same + s)) + ext_jj + pulse proj_j of
-// every matrix, DIAG_T trajectories per CTA: one read of row k of U and V serves their 2
-// DIAG_T matrices.  Inside the stage kernel the same sums were one thread's chain of 2 n
-// loads per site before the matrix's epilogue could begin: half of the kernel's time at
-// n = 256 (1440 -> 1150 us per stage and 2048 matrices, and 70 us here).
+// Delta_jj (diag_site) of every matrix with dense Coulomb rows, DIAG_T trajectories per CTA: one
+// read of row k of U and V serves their 2 DIAG_T matrices.  Inside the stage kernel the same sums
+// are one thread's chain of n terms each per site before the matrix's epilogue can begin, hidden
+// behind the MMAs only while few matrices follow one another in a CTA.  Four steps, n = 256, BF16x3,
+// inside against here: 200 matrices 2.45 and 2.96 ms, 400 3.94 and 4.17, 600 6.42 and 6.48, 1024 9.46
+// and 9.01, 2048 19.5 and 17.5.  Rows with few entries stay inside at every size.
 constexpr int DIAG_T = 4;
 __global__ void __launch_bounds__(NP) k_dense_diag(DenseArgs a)
 {
@@ -425,38 +460,27 @@ __global__ void __launch_bounds__(NP) k_dense_diag(DenseArgs a)
     float u[2 * DIAG_T], v[2 * DIAG_T];
 #pragma unroll
     for (int q = 0; q < 2 * DIAG_T; ++q) u[q] = v[q] = 0.f;
-    if (a.Ud) {
-        // U and V are symmetric: thread j walks column j, the warp reads row k
+    // U and V are symmetric: thread j walks column j, the warp reads row k
 #pragma unroll 8
-        for (int k = 0; k < a.n; ++k) {
-            const float uk = __ldg(a.Ud + (size_t)k * NP + j), vk = __ldg(a.Vd + (size_t)k * NP + j);
+    for (int k = 0; k < a.n; ++k) {
+        const float uk = __ldg(a.Ud + (size_t)k * NP + j), vk = __ldg(a.Vd + (size_t)k * NP + j);
 #pragma unroll
-            for (int q = 0; q < 2 * DIAG_T; ++q) {
-                u[q] = fmaf(uk, nd[q ^ 1][k], u[q]);
-                v[q] = fmaf(vk, nd[q][k], v[q]);
-            }
+        for (int q = 0; q < 2 * DIAG_T; ++q) {
+            u[q] = fmaf(uk, nd[q ^ 1][k], u[q]);
+            v[q] = fmaf(vk, nd[q][k], v[q]);
         }
-    } else if (sy.coul != 0 && j < a.n) {
-        for (int x = sy.up[j]; x < sy.up[j + 1]; ++x)
-#pragma unroll
-            for (int q = 0; q < 2 * DIAG_T; ++q) u[q] = fmaf(sy.uv[x], nd[q ^ 1][sy.uk[x]], u[q]);
-        if (sy.coul == 2)
-            for (int x = sy.vp[j]; x < sy.vp[j + 1]; ++x)
-#pragma unroll
-                for (int q = 0; q < 2 * DIAG_T; ++q) v[q] = fmaf(sy.vv[x], nd[q][sy.vk[x]], v[q]);
     }
 #pragma unroll
     for (int q = 0; q < 2 * DIAG_T; ++q) {
         if (q >= nm) continue;
         float d = 0.f;
         if (j < a.n) {
-            d = sy.tdiag[j];
-            if (sy.coul != 0) d += u[q];
+            d = sy.tdiag[j] + u[q];
             if (sy.coul == 2) d += v[q];
             if (sy.has_ext) d += sy.ediag[j];
             if (sy.n_bins > 0) d += a.pulse * sy.proj[j];
         }
-        a.dvec[(size_t)(m0 + q) * NP + j] = d;
+        a.dvec[(size_t)(m0 + q) * 2 * PLANE + j] = d;
     }
 }
 
@@ -526,7 +550,8 @@ __global__ void k_dense_pack(const float* __restrict__ X, int n, int M, cplx<R>*
 
 // One snapshot record straight from the planes, a trajectory per CTA: the hopping and
 // potential rows as one sweep of each spin's real plane against tM in the same order (16-byte
-// loads, FP64 sums), the Coulomb rows from dense U and V with the threads along a row.  The
+// loads, FP64 sums; up to the last row of blocks that holds a site), the Coulomb rows from dense U
+// and V with the threads along a row.  The
 // packed copy and the one-thread-per-site index lists it replaces took 1.76 ms per snapshot
 // at n = 256, 1024 trajectories; this takes 0.28 ms.
 constexpr int REC_NT = 256;
@@ -551,13 +576,14 @@ __global__ void __launch_bounds__(REC_NT) k_dense_record(DenseRecordArgs a)
     if (!a.do_en) return;
     __syncthreads();
     double e[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+    const int nq = (a.n + 31) / 32 * (32 * NP / 4);      // the rows of blocks that hold sites
     for (int s = 0; s < 2; ++s) {
         const float4* x4 = reinterpret_cast<const float4*>(Xu + (size_t)s * 2 * PLANE);
         const float4* t4 = reinterpret_cast<const float4*>(a.Tt);
         const float4* v4 = reinterpret_cast<const float4*>(a.Et);
         double t = 0.0, p = 0.0;
 #pragma unroll 4
-        for (int q = tid; q < (int)(PLANE / 4); q += REC_NT) {
+        for (int q = tid; q < nq; q += REC_NT) {
             const float4 x = x4[q], h = __ldg(t4 + q);
             t += (double)x.x * (double)h.x + (double)x.y * (double)h.y + (double)x.z * (double)h.z + (double)x.w * (double)h.w;
             if (a.Et) {
@@ -625,7 +651,7 @@ cudaError_t configure()
 
 cudaError_t launch_stage(const DenseArgs& a, int grid, bool tf32, cudaStream_t st)
 {
-    k_dense_diag<<<(a.M + 2 * DIAG_T - 1) / (2 * DIAG_T), NP, 0, st>>>(a);
+    if (a.dvec) k_dense_diag<<<(a.M + 2 * DIAG_T - 1) / (2 * DIAG_T), NP, 0, st>>>(a);
     if (tf32) k_dense_stage<true><<<grid, NTHREADS, stage_smem_bytes(), st>>>(a);
     else k_dense_stage<false><<<grid, NTHREADS, stage_smem_bytes(), st>>>(a);
     return cudaGetLastError();

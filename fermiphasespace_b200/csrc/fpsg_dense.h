@@ -43,7 +43,10 @@ struct DenseArgs {
     DevSys<float> sys;           // diagonal terms (tM_jj, Hartree rows, potential, pulse projection)
     const float* Ud;             // dense U, V ([NP][NP], zero-padded) for long-range Coulomb, else null
     const float* Vd;
-    float* dvec;                 // [M][NP] Delta_jj of the stage input (k_dense_diag)
+    // Delta_jj of the stage input by matrix, 2 NP NP floats apart (k_dense_diag; `out` will do, the
+    // stage kernel takes a matrix's values before it writes there); null: the stage kernel forms them
+    float* dvec;
+    bool prefetch;               // read ahead into L2 (enough CTAs at work for DRAM to be the limit)
     float pulse;                 // pulse amplitude x envelope at the stage time
     unsigned* err;
     // test hook (FPSG_FLAG_TEST_EXPIRE_WAIT): > 0 makes one thread wait, with this
