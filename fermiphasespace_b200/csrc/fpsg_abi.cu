@@ -274,7 +274,7 @@ struct TableBlock {
     {
         const size_t bytes = sizeof(T) * std::max<size_t>(v.size(), 1);
         pieces.push_back({v.data(), sizeof(T) * v.size(), total, (void**)dst});
-        total += (bytes + 255) & ~size_t(255);
+        total += (bytes + 15) & ~size_t(15);
     }
     int upload(fpsg_ctx* ctx, void** block)
     {
@@ -297,7 +297,7 @@ void free_tables(fpsg_ctx* ctx, DevTables<R>& t)
 }
 
 template <typename R>
-int build_tables(fpsg_ctx* ctx, DevTables<R>& t)
+int build_tables(fpsg_ctx* ctx, DevTables<R>& t, bool dense)
 {
     const int n = ctx->n;
     std::vector<int> hp(1, 0), hk, up(1, 0), uk, vp(1, 0), vk;
@@ -481,7 +481,7 @@ int build_tables(fpsg_ctx* ctx, DevTables<R>& t)
     // dense rows of U (and V) where most of their entries are nonzero
     std::vector<R> ud, vd;
     const size_t nn = (size_t)n * n;
-    if (ctx->coul != FPSG_COULOMB_NULL && 2 * (uk.size() + (ctx->coul == FPSG_COULOMB_DISTANCE ? vk.size() : 0)) >= nn && n > 4) {
+    if (dense && ctx->coul != FPSG_COULOMB_NULL && 2 * (uk.size() + (ctx->coul == FPSG_COULOMB_DISTANCE ? vk.size() : 0)) >= nn && n > 4) {
         ud.resize(nn);
         vd.resize(nn);
         for (size_t q = 0; q < nn; ++q) { ud[q] = (R)ctx->U[q]; vd[q] = (R)ctx->V[q]; }
@@ -500,6 +500,23 @@ int build_tables(fpsg_ctx* ctx, DevTables<R>& t)
     if (rc) return rc;
     t.pat.mask = d_mask;
     return FPSG_OK;
+}
+
+// Both precisions' tables, without the dense Coulomb rows where those do not fit: the index lists
+// say the same.
+int build_all_tables(fpsg_ctx* ctx)
+{
+    int rc = FPSG_OK;
+    for (const bool dense : {true, false}) {
+        free_tables(ctx, ctx->t64);
+        free_tables(ctx, ctx->t32);
+        if (!dense) trim_pool(ctx);         // a block of the larger tables would be taken for the smaller ones
+        rc = build_tables<double>(ctx, ctx->t64, dense);
+        if (!rc) rc = build_tables<float>(ctx, ctx->t32, dense);
+        if (rc != FPSG_ERR_OOM) break;
+    }
+    if (!rc) ctx->err.clear();
+    return rc;
 }
 
 template <typename R>
@@ -2555,6 +2572,7 @@ int fpsg_set_system(fpsg_ctx* ctx, int n, const double* tM, const double* U, con
         check_real_symmetric(V, n, "V", why) || (!extpot_is_null && check_real_symmetric(extpot, n, "extpot", why)))
         return fail(ctx, FPSG_ERR_UNSUPPORTED, why + " (the engine needs real symmetric inputs)");
     if (cudaSetDevice(ctx->device) != cudaSuccess) return fail(ctx, FPSG_ERR_CUDA, "cudaSetDevice");
+    ctx->sys_set = false;       // until every table is there
     free_tables(ctx, ctx->t64);
     free_tables(ctx, ctx->t32);
     trelease(ctx, ctx->order_block); ctx->order_block = nullptr;
@@ -2586,8 +2604,7 @@ int fpsg_set_system(fpsg_ctx* ctx, int n, const double* tM, const double* U, con
     TableBlock tb;
     tb.add(&ctx->pij, pij); tb.add(&ctx->res_order, ro); tb.add(&ctx->pair_order, po);
     if ((rc = tb.upload(ctx, &ctx->order_block))) return rc;
-    if ((rc = build_tables<double>(ctx, ctx->t64))) return rc;
-    if ((rc = build_tables<float>(ctx, ctx->t32))) return rc;
+    if ((rc = build_all_tables(ctx))) return rc;
     ctx->sys_set = true;
     return FPSG_OK;
 }
@@ -2610,11 +2627,12 @@ int fpsg_set_pulse(fpsg_ctx* ctx, int n_bins, const double* amp, double bin_widt
         int rc;
         if ((rc = upload(ctx, &ctx->d_amp, ctx->amp))) return rc;
     }
+    ctx->sys_set = false;       // until every table is there
     free_tables(ctx, ctx->t64);
     free_tables(ctx, ctx->t32);
     int rc;
-    if ((rc = build_tables<double>(ctx, ctx->t64))) return rc;
-    if ((rc = build_tables<float>(ctx, ctx->t32))) return rc;
+    if ((rc = build_all_tables(ctx))) return rc;
+    ctx->sys_set = true;
     return FPSG_OK;
 }
 
