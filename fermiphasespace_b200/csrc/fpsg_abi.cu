@@ -1572,7 +1572,8 @@ int grad_impl(fpsg_ctx* ctx, double dt, int S, int Tp, int C, double* loss_out, 
         // needs no memory that it does not have: one chunk, without a look at the free memory, a
         // driver call that has been seen to take tens of milliseconds on a busy host.  The block
         // is set aside, so that no other request takes or frees it.
-        const bool fits = bi >= 0 && !ctx->mem_cap && ctx->grad_keep < 0 &&
+        const bool fits = bi >= 0 && !ctx->mem_cap &&
+                          (ctx->grad_keep < 0 || (size_t)ctx->grad_keep >= (size_t)Ball * per_keep) &&
                           ctx->pool[bi].bytes >= (size_t)Ball * per_keep &&
                           pooled - ctx->pool[bi].bytes >= (size_t)Ball * per_tmp;
         if (fits) {
