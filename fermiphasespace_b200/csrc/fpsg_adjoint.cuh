@@ -395,7 +395,9 @@ __host__ __device__ __forceinline__ size_t vjp_seg_smem(int n, int ne, int n_bin
 // Bound by the chain of each stage (shared-memory latency and the barriers; 29 % of the FP32
 // rate).  Measured per segment: 8x8 grid, FP32, 1024 trajectories, 16 steps: 3.07 ms with
 // column entries, 3.03 with the pattern; 5x5 grid, FP64, 300 trajectories, ten steps: 0.545 ms
-// with column entries and 512 threads, 0.30 with the pattern and 128.
+// with column entries and 512 threads, 0.30 with the pattern and 128.  What the entries cost went
+// into spills at the 64 registers of XS: FP32, 512 threads, 84 bytes of stores and 172 of loads per
+// thread with the pattern, 12 and 20 with entries; FP64, 128 threads, 148 and 344 against 104 and 156.
 template <typename R, int NT, int EPT, int P, bool XS = false>
 __global__ void __launch_bounds__(NT, (XS ? 1024 : 512) / NT) k_vjp_segment(VjpSegArgs<R> a)
 {

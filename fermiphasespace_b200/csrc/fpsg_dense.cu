@@ -21,8 +21,9 @@
 //
 // One launch = one RK stage of every spin matrix.  Persistent CTAs (one per SM),
 // warp-specialised:
-//   warps 0-15  epilogue: per plane read
-//               the accumulator from tensor memory and write
+//   warps 0-15  epilogue: the Hartree diagonal d of the matrix (formed here, or read
+//               where k_dense_diag has formed it), then per plane read the
+//               accumulator from tensor memory and write
 //               out = a0 P0 + a1 P1 + ax X + hk k (the 3/8 RK rule in terms of
 //               stored stage inputs)
 //   warps 16-23 producers: stage X chunks (256 rows x 32 columns) into shared
@@ -553,7 +554,7 @@ __global__ void k_dense_pack(const float* __restrict__ X, int n, int M, cplx<R>*
 // loads, FP64 sums; up to the last row of blocks that holds a site), the Coulomb rows from dense U
 // and V with the threads along a row.  The
 // packed copy and the one-thread-per-site index lists it replaces took 1.76 ms per snapshot
-// at n = 256, 1024 trajectories; this takes 0.28 ms.
+// at n = 256, 1024 trajectories; this takes 0.23 ms.
 constexpr int REC_NT = 256;
 __global__ void __launch_bounds__(REC_NT) k_dense_record(DenseRecordArgs a)
 {

@@ -17,6 +17,8 @@
 // entries 0 (24), state 4 (4), diagonal terms 2 (4), stores 8 (8): 42 against 78.
 // FP32 arithmetic runs on the two-wide instructions, a complex number per instruction.
 // 10x10 grid, FP32, 16384 trajectories x 41 steps: 189.0 -> 113.5 ms
+// The FP64 instances spill at 128 registers, the fullest, <256, 5, split>, 600 bytes of stores and
+// 388 of loads per thread; the FP32 ones that forward runs take do not.
 //
 // Otherwise the kernel is k_resident: M stacked spin matrices per CTA (one spin per CTA
 // of a 2-CTA cluster in split mode), X double-buffered in shared memory, the state at the
@@ -602,7 +604,9 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_pair(ResArgs<R> a)
 // state and stores it, so no stage output is held across the barrier.  FP64 keeps k1 and k2
 // themselves and forms A = k1 - k2 and Bc = k1 + 3 k2 one stage later, by the same
 // operations: bit-identical to the oracle.
-// 10x10 grid, FP64, 4096 trajectories x 41 steps: 134.7 -> 77.0 ms
+// 10x10 grid, FP64, 4096 trajectories x 41 steps: 134.7 -> 76 ms
+// Spilled per thread, stores / loads in bytes: FP64 with five slots 284 / 364 (n = 100), with four 96
+// / 136; FP32 with eight 296 / 68, with eleven (MEMC) 304 / 532; FP64 with three and FP32 with six none.
 __host__ __device__ __forceinline__ int packed_col(int c, int D) { return (c * (c + 2 * D + 1)) >> 1; }
 
 // C(j + o) - C(j) = o j + up[s], C(j - o) - C(j) = dn[s] - o j for the offsets o of a
