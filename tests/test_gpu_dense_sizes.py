@@ -25,8 +25,9 @@ def system(n, coulomb, ext=True):
     return T, U, V, X, occ
 
 
+@pytest.mark.parametrize("prec", [E.PREC_SPLIT_BF16X3, E.PREC_SPLIT_TF32X3])
 @pytest.mark.parametrize("coulomb", [E.COUL_ONSITE, E.COUL_DISTANCE])
-def test_a_trajectory_does_not_depend_on_the_others(coulomb):
+def test_a_trajectory_does_not_depend_on_the_others(coulomb, prec):
     """One matrix per CTA, several, and more than five (own launch for dense rows): the same sums in
     the same order, so the same bits."""
     T, U, V, X, occ = system(30, coulomb)
@@ -35,7 +36,7 @@ def test_a_trajectory_does_not_depend_on_the_others(coulomb):
     states = []
     for B in (3, 75, 400):
         eng.sample(B, 5, occ, 1.0 - occ)
-        eng.advance(E.METHOD_FTWA, E.PREC_SPLIT_BF16X3, 0.005, 1, 3)
+        eng.advance(E.METHOD_FTWA, prec, 0.005, 1, 3)
         states.append(eng.get_state()[:3])
     eng.close()
     assert np.array_equal(states[0], states[1]) and np.array_equal(states[0], states[2])
